@@ -206,9 +206,10 @@ int plume_multigrid(const PlumeLevel* levels, int32_t level_count, int32_t cycle
 
 /* Pressure-solve strategy (no reference counterpart; results do not depend on it): levels with at least
  * `tiled_min_cells` cells sweep in shared-memory tiles (one launch per sweep), smaller levels one colour per
- * launch; the first level with at most `bottom_max_cells` cells and all coarser ones run in one launch:
- * bottom_kind 1 an 8-CTA thread-block cluster (levels split in x-slabs over the CTAs' shared memory), 0 one
- * 1024-thread block; at most 200 KiB of shared memory per CTA. Process-wide; defaults 2^40, 2048, 0. */
+ * launch; the first level with at most `bottom_max_cells` cells and all coarser ones run in one launch of one
+ * thread-block cluster, in its shared memory: bottom_kind 0 up to 16 CTAs, with the levels of up to about 10^5
+ * cells above the bottom in the same launch (levels of at most `bottom_max_cells` in one CTA; 0: every level by
+ * launches of its own); bottom_kind 1 8 CTAs from the bottom level on. Process-wide; defaults 2^40, 2048, 0. */
 int plume_tune_solver(long long tiled_min_cells, long long bottom_max_cells, int32_t bottom_kind);
 /* The current pressure-solve strategy (the three values plume_tune_solver sets). */
 int plume_solver_tuning(long long* tiled_min_cells, long long* bottom_max_cells, int32_t* bottom_kind);

@@ -8,12 +8,11 @@
 //   - the residual, its restriction to the coarse level and the zeroing of the coarse pressure are one
 //     launch (k_residual_restrict);
 //   - prolongation is folded into the first post-smoothing sweep (the tile loads q + prolong(coarse));
-//   - every level from the first of at most 2048 cells down to the coarsest solve runs in one launch: one
-//     1024-thread block with all its arrays in shared memory (k_block_solve), or, selectable, one 8-CTA
-//     thread-block cluster with the larger levels split in x-slabs over distributed shared memory
-//     (k_cluster_solve).
-#include <cooperative_groups.h>
-
+//   - the small levels run in one launch (cluster_solve.cu): from the first of at most cluster_max_cells cells
+//     down, in the shared memory of a 16-CTA thread-block cluster, those of at most 2048 cells in one CTA of it.
+//     When that covers the whole hierarchy, all cycles are that one launch;
+//   - the defect-correction solve's cycles, whose coarsest level is swept in double, run the levels of at most
+//     2048 cells in one 1024-thread block instead (k_block_solve).
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>
@@ -21,6 +20,7 @@
 #include <mutex>
 #include <vector>
 
+#include "cluster_solve.cuh"
 #include "poisson.cuh"
 
 namespace plume {
@@ -33,15 +33,13 @@ constexpr int COARSEST_SWEEPS = 20;  // multigrid.py:24-33
 constexpr int COARSEST_SWEEPS_PER_CELL = 4;
 constexpr int BOTTOM_THREADS = 1024;
 constexpr int BOTTOM_MAX_LEVELS = 8;
+constexpr long SINGLE_MAX_CELLS = 1024;  // bottom kind 1: larger levels are spread over its 8 CTAs
 constexpr int BOTTOM_WARP_PAIRS = 128;  // levels with at most this many cell pairs per colour run on one warp
 // Per-level strategy (set by plume_tune_solver): levels of at least g_tiled_min_cells cells sweep in tiles,
 // smaller ones one colour per launch; the first level of at most g_bottom_max_cells cells and everything
-// below it runs in one block.
+// below it runs in one launch (coarse_plan).
 static long g_tiled_min_cells = 1L << 40;  // measured: per-colour sweeps win while the levels fit in L2
-// Measured on B200 (128x192x128 and 256x384x256 hierarchies, 4 V-cycles): the one-block solve beats the 8-CTA
-// cluster solve, whose passes are bound by barrier latency, and starting it at the first level of at most
-// 2048 cells (rather than 8192) saves 9% of the solve: a 16x24x16 level sweeps faster as per-colour launches
-// across the GPU than inside one block on one SM.
+// Levels of at most this many cells run in one CTA (plume_tune_solver's bottom_max_cells).
 static long g_bottom_max_cells = 2048;
 // The top level runs in colour-split storage (given caller scratch) when it has at least this many cells
 // (plume_tune_split): levels whose q and rhs do not fit in L2. Measured on B200 at 256x384x256, 4 V-cycles: the
@@ -49,7 +47,23 @@ static long g_bottom_max_cells = 2048;
 // 109 us, residual and restriction about 110 against 107 us, plus 0.15 ms of layout conversions per solve); at
 // 128x192x128, whose levels fit in L2, split is slower (0.97 against 0.78 ms).
 static long g_split_min_cells = 1L << 23;
-static int g_bottom_kind = 0;  // 0: the one-block solve, 1: the cluster solve
+static int g_bottom_kind = 0;  // 0: levels above the bottom join its launch in a 16-CTA cluster; 1: an 8-CTA cluster from the bottom
+// Levels above the bottom join its launch (bottom kind 0) up to this many cells. A colour pass of a level costs a launch
+// of its own about 2 us in a graph, and in the cluster 0.6 us and 0.8 us more per 110 thousand cells; where the cluster
+// starts below the top level, each cycle also loads and stores its first level (3 us). Measured on B200, 4 cycles, with
+// the level at stake in the cluster and as launches of its own: 32x48x32 below a 64x96x64 grid 270 and 284 us,
+// 40x60x40 below 160x240x160 1147 and 1133 us, 48x72x48 below 96x144x96 468 and 439 us; the top level 48x48x48 207 and
+// 217 us, 48x72x48 236 and 229 us; overhanging cells cost the launches more: 38x57x46 below 75x113x91 455 and 482 us.
+// PLUME_CLUSTER_MAX_CELLS overrides both limits (for measurements).
+static long cluster_max_cells(const PlumeGridInfo& info, bool top) {
+  static const long set = [] {
+    const char* v = getenv("PLUME_CLUSTER_MAX_CELLS");
+    return v ? atol(v) : 0L;
+  }();
+  if (set) return set;
+  const bool overhangs = info.fill_hi[0] != 1.0f || info.fill_hi[1] != 1.0f || info.fill_hi[2] != 1.0f;
+  return top || overhangs ? 120000 : 60000;
+}
 constexpr size_t BOTTOM_MAX_SMEM = 200 * 1024;
 
 // The solve's kernels are launched with programmatic dependent launch: each may be scheduled while the
@@ -638,291 +652,7 @@ __global__ void k_prolong_add_split8(Dims coarse, Dims fine, int H, const float*
   }
 }
 
-// ---- the cluster coarse solve --------------------------------------------------------------------------------
-// Every level from `first` down runs in one launch of one thread-block cluster (CLUSTER CTAs, one per SM).
-// A level above SINGLE_MAX_CELLS cells is split into slabs of whole x-planes, one slab per CTA, held in that
-// CTA's shared memory; a CTA reads its neighbours' boundary planes through distributed shared memory and
-// the cluster barrier separates the passes. Smaller levels live in CTA 0 alone and run with block or warp
-// barriers while the other CTAs wait at the next cluster barrier. Every cell gets exactly the reference's
-// update; only where the values are stored differs.
-
-constexpr int CLUSTER = 8;
-constexpr long SINGLE_MAX_CELLS = 1024;
-
-struct LevelView {
-  PlumeGridInfo info;
-  float* q;        // global arrays (loaded for the first level, written back for all)
-  float* rhs;
-  int planes;      // x-planes per CTA (the whole level when single)
-  int single;      // 1: the level lives in CTA 0
-  int offset;      // shared-memory float offset of the level's q block; its rhs block follows
-};
-
-struct ClusterArgs {
-  int count;
-  int sweeps;
-  LevelView lv[BOTTOM_MAX_LEVELS];
-};
-
-namespace cg = cooperative_groups;
-
-struct ClusterCtx {
-  cg::cluster_group cluster;
-  float* smem;
-  int rank;
-};
-
-// The CTA holding plane i (no division: slabs are `planes` planes long, CLUSTER of them).
-__device__ __forceinline__ int owner_of(const LevelView& L, int i) {
-  if (L.single) return 0;
-  int owner = 0;
-#pragma unroll
-  for (int r = 1; r < CLUSTER; ++r) owner += i >= r * L.planes;
-  return owner;
-}
-
-__device__ __forceinline__ int local_index(const LevelView& L, int owner, int i, int j, int k, bool rhs) {
-  const int n1 = L.info.dims[1], n2 = L.info.dims[2];
-  const int li = L.single ? i : i - owner * L.planes;
-  return L.offset + (rhs ? L.planes * n1 * n2 : 0) + (li * n1 + j) * n2 + k;
-}
-
-// q (or rhs) of a cell, read from whichever CTA holds its plane: a shared-memory load when it is this CTA.
-__device__ __forceinline__ float cell_load(const ClusterCtx& c, const LevelView& L, int i, int j, int k, bool rhs) {
-  const int owner = owner_of(L, i);
-  const int idx = local_index(L, owner, i, j, k, rhs);
-  if (owner == c.rank) return c.smem[idx];
-  return *c.cluster.map_shared_rank(c.smem + idx, owner);
-}
-
-__device__ __forceinline__ void cell_store(const ClusterCtx& c, const LevelView& L, int i, int j, int k, bool rhs,
-                                           float value) {
-  const int owner = owner_of(L, i);
-  const int idx = local_index(L, owner, i, j, k, rhs);
-  if (owner == c.rank) c.smem[idx] = value;
-  else *c.cluster.map_shared_rank(c.smem + idx, owner) = value;
-}
-
-// The x-planes [lo, hi) a CTA works on in a pass over level L: its own slab, or everything in CTA 0.
-__device__ __forceinline__ void my_planes(const ClusterCtx& c, const LevelView& L, int& lo, int& hi) {
-  const int n0 = L.info.dims[0];
-  if (L.single) {
-    lo = 0;
-    hi = c.rank == 0 ? n0 : 0;
-    return;
-  }
-  lo = imin_(c.rank * L.planes, n0);
-  hi = imin_(lo + L.planes, n0);
-}
-
-// One pass of cells of one colour over the planes [lo, hi), `threads` threads from thread 0.
-template <class Update>
-__device__ __forceinline__ void for_colour(const LevelView& L, int lo, int hi, int color, int threads, Update update) {
-  const int n1 = L.info.dims[1], n2 = L.info.dims[2];
-  const int pairs_k = (n2 + 1) / 2;
-  const int per_plane = n1 * pairs_k;
-  const int pairs = (hi - lo) * per_plane;
-  for (int p = threadIdx.x; p < pairs; p += threads) {
-    const int a = p / per_plane, rem = p - a * per_plane, j = rem / pairs_k, kp = rem - j * pairs_k;
-    const int i = lo + a;
-    const int k = 2 * kp + ((i + j + color) & 1);
-    if (k < n2) update(i, j, k);
-  }
-}
-
-// `sweeps` red-black sweeps of level L. Neighbours in the same x-plane are always this CTA's; the x-1 and
-// x+1 planes come from the neighbouring CTAs' shared memory at the slab edges. A single level small enough
-// for one warp syncs at warp level.
-__device__ void cluster_smooth(const ClusterCtx& c, const LevelView& L, int sweeps, float relaxation) {
-  const PlumeGridInfo& info = L.info;
-  const bool uniform = is_uniform(info);
-  const float ghost = ghost_coupling(info);
-  const int n0 = info.dims[0], n1 = info.dims[1], n2 = info.dims[2];
-  const int plane = n1 * n2;
-  int lo, hi;
-  my_planes(c, L, lo, hi);
-  float* q = c.smem + L.offset;               // this CTA's planes [lo, hi), then their rhs
-  const float* rhs = q + L.planes * plane;
-  const float* q_prev = (!L.single && lo > 0 && lo < hi) ? c.cluster.map_shared_rank(q + (L.planes - 1) * plane, c.rank - 1)
-                                                         : nullptr;
-  const float* q_next = (!L.single && hi < n0 && lo < hi) ? c.cluster.map_shared_rank(q, c.rank + 1) : nullptr;
-  auto update = [&](int i, int j, int k) {
-    const int idx = (i - lo) * plane + j * n2 + k;
-    auto load = [&](int a, int b, int cc) {
-      if (a == i) return q[idx + (b - j) * n2 + (cc - k)];
-      if (a == i - 1) return i - 1 >= lo ? q[idx - plane] : q_prev[j * n2 + k];
-      return i + 1 < hi ? q[idx + plane] : q_next[j * n2 + k];
-    };
-    float out;
-    if (relax_cell(uniform, info, ghost, i, j, k, q[idx], rhs[idx], relaxation, load, out)) q[idx] = out;
-  };
-  const int pairs_k = (n2 + 1) / 2;
-  const int per_plane = n1 * pairs_k;
-  const int t = threadIdx.x;
-  auto colour_pass = [&](int color, int threads) {
-    if (per_plane <= threads && (hi - lo) * per_plane > threads) {  // each thread owns a column of every plane
-      if (t < per_plane) {
-        const int j = t / pairs_k, kp = t - j * pairs_k;
-        for (int i = lo; i < hi; ++i) {
-          const int k = 2 * kp + ((i + j + color) & 1);
-          if (k < n2) update(i, j, k);
-        }
-      }
-    } else {
-      for_colour(L, lo, hi, color, threads, update);
-    }
-  };
-  if (L.single) {
-    const int pairs = n0 * per_plane;
-    const bool one_warp = pairs <= BOTTOM_WARP_PAIRS;
-    if (c.rank == 0 && (!one_warp || t < 32)) {
-      for (int s = 0; s < sweeps; ++s)
-        for (int color = 0; color < 2; ++color) {
-          if (one_warp) {
-            for_colour(L, lo, hi, color, 32, update);
-            __syncwarp();
-          } else {
-            colour_pass(color, BOTTOM_THREADS);
-            __syncthreads();
-          }
-        }
-    }
-    if (c.rank == 0) __syncthreads();  // the rest of CTA 0 waits for the warp that did the work
-    return;
-  }
-  for (int s = 0; s < sweeps; ++s)
-    for (int color = 0; color < 2; ++color) {
-      colour_pass(color, BOTTOM_THREADS);
-      c.cluster.sync();
-    }
-}
-
-// residual + restriction + zero coarse pressure (multigrid.py:36-60, :143) from F into C. Coarse planes are
-// shared out over the CTAs by slab; each writes into whichever CTA holds the coarse plane.
-__device__ void cluster_restrict(const ClusterCtx& c, const LevelView& F, const LevelView& C, bool single_only) {
-  const PlumeGridInfo& info = F.info;
-  const Dims fd = dims_of(info), cd = dims_of(C.info);
-  const bool uniform = is_uniform(info);
-  const float ghost = ghost_coupling(info);
-  auto load = [&](int a, int b, int k) { return cell_load(c, F, a, b, k, false); };
-  int lo, hi;
-  if (single_only) {
-    lo = 0;
-    hi = c.rank == 0 ? cd.n0 : 0;
-  } else {
-    const int per = (cd.n0 + CLUSTER - 1) / CLUSTER;
-    lo = imin_(c.rank * per, cd.n0);
-    hi = imin_(lo + per, cd.n0);
-  }
-  const int cells = (hi - lo) * cd.n1 * cd.n2;
-  for (int idx = threadIdx.x; idx < cells; idx += BOTTOM_THREADS) {
-    const int a = idx / (cd.n1 * cd.n2), rem = idx - a * (cd.n1 * cd.n2), j = rem / cd.n2, k = rem - j * cd.n2;
-    const int i = lo + a;
-    float total = 0.0f, count = 0.0f;
-    for (int di = 0; di < 2; ++di)
-      for (int dj = 0; dj < 2; ++dj)
-        for (int dk = 0; dk < 2; ++dk) {
-          const int fi = 2 * i + di, fj = 2 * j + dj, fk = 2 * k + dk;
-          if (fi < fd.n0 && fj < fd.n1 && fk < fd.n2) {
-            total = total + residual_cell(uniform, info, ghost, fi, fj, fk, cell_load(c, F, fi, fj, fk, false),
-                                          cell_load(c, F, fi, fj, fk, true), load);
-            count = count + 1.0f;
-          }
-        }
-    cell_store(c, C, i, j, k, true, total / count);
-    cell_store(c, C, i, j, k, false, 0.0f);
-  }
-}
-
-// prolong_add_kernel (multigrid.py:63-68): each CTA adds the coarse correction to the fine planes it holds.
-__device__ void cluster_prolong(const ClusterCtx& c, const LevelView& F, const LevelView& C) {
-  const Dims fd = dims_of(F.info), cd = dims_of(C.info);
-  int lo, hi;
-  my_planes(c, F, lo, hi);
-  const int cells = (hi - lo) * fd.n1 * fd.n2;
-  for (int idx = threadIdx.x; idx < cells; idx += BOTTOM_THREADS) {
-    const int a = idx / (fd.n1 * fd.n2), rem = idx - a * (fd.n1 * fd.n2), j = rem / fd.n2, k = rem - j * fd.n2;
-    const int i = lo + a;
-    const F3 g = prolong_point(i, j, k);  // sample_index_space (sample.py:10-29) on the coarse level
-    const float x = clampf_(g[0], 0.0f, (float)(cd.n0 - 1)), y = clampf_(g[1], 0.0f, (float)(cd.n1 - 1)),
-                z = clampf_(g[2], 0.0f, (float)(cd.n2 - 1));
-    const int i0 = (int)x, j0 = (int)y, k0 = (int)z;
-    const int i1 = imin_(i0 + 1, cd.n0 - 1), j1 = imin_(j0 + 1, cd.n1 - 1), k1 = imin_(k0 + 1, cd.n2 - 1);
-    const float tx = x - (float)i0, ty = y - (float)j0, tz = z - (float)k0;
-    auto cq = [&](int a2, int b2, int k2) { return cell_load(c, C, a2, b2, k2, false); };
-    const float c00 = lerpf_(cq(i0, j0, k0), cq(i1, j0, k0), tx);
-    const float c10 = lerpf_(cq(i0, j1, k0), cq(i1, j1, k0), tx);
-    const float c01 = lerpf_(cq(i0, j0, k1), cq(i1, j0, k1), tx);
-    const float c11 = lerpf_(cq(i0, j1, k1), cq(i1, j1, k1), tx);
-    const int at_q = local_index(F, c.rank, i, j, k, false);  // a plane this CTA holds
-    c.smem[at_q] = c.smem[at_q] + lerpf_(lerpf_(c00, c10, ty), lerpf_(c01, c11, ty), tz);
-  }
-}
-
-// A barrier for the level just processed: the cluster for split levels, CTA 0's block for single ones.
-__device__ __forceinline__ void level_barrier(const ClusterCtx& c, bool cluster_wide) {
-  if (cluster_wide) c.cluster.sync();
-  else if (c.rank == 0) __syncthreads();
-}
-
-__global__ void __launch_bounds__(BOTTOM_THREADS) k_cluster_solve(ClusterArgs b) {
-  extern __shared__ float smem[];
-  ClusterCtx c{cg::this_cluster(), smem, (int)cg::this_cluster().block_rank()};
-  {  // the first level's pressure and right-hand side, each CTA its planes
-    const LevelView& L = b.lv[0];
-    int lo, hi;
-    my_planes(c, L, lo, hi);
-    const int n1 = L.info.dims[1], n2 = L.info.dims[2];
-    const int cells = (hi - lo) * n1 * n2;
-    const long base = (long)lo * n1 * n2;
-    float* q = smem + L.offset;
-    float* rhs = q + L.planes * n1 * n2;
-    for (int idx = threadIdx.x; idx < cells; idx += BOTTOM_THREADS) {
-      q[idx] = L.q[base + idx];
-      rhs[idx] = L.rhs[base + idx];
-    }
-  }
-  c.cluster.sync();
-  const int last = b.count - 1;
-  for (int l = 0; l < last; ++l) {  // down: smooth, then residual and restriction into the next level
-    const LevelView& F = b.lv[l];
-    const LevelView& C = b.lv[l + 1];
-    cluster_smooth(c, F, b.sweeps, 1.0f);
-    cluster_restrict(c, F, C, F.single != 0);
-    level_barrier(c, F.single == 0);
-  }
-  {  // the coarsest solve (multigrid.py:132-136)
-    const LevelView& L = b.lv[last];
-    const int longest = imax_(L.info.dims[0], imax_(L.info.dims[1], L.info.dims[2]));
-    cluster_smooth(c, L, imax_(COARSEST_SWEEPS, COARSEST_SWEEPS_PER_CELL * longest), 1.5f);
-  }
-  for (int l = last - 1; l >= 0; --l) {  // up: prolong the coarse correction, smooth
-    const LevelView& F = b.lv[l];
-    const LevelView& C = b.lv[l + 1];
-    if (F.single == 0 && C.single) c.cluster.sync();  // the single part is done before its correction is read
-    cluster_prolong(c, F, C);
-    level_barrier(c, F.single == 0);
-    cluster_smooth(c, F, b.sweeps, 1.0f);
-  }
-  c.cluster.sync();
-  for (int l = 0; l < b.count; ++l) {  // every level's pressure (and the coarse right-hand sides) back out
-    const LevelView& L = b.lv[l];
-    int lo, hi;
-    my_planes(c, L, lo, hi);
-    const int n1 = L.info.dims[1], n2 = L.info.dims[2];
-    const int cells = (hi - lo) * n1 * n2;
-    const long base = (long)lo * n1 * n2;
-    const float* q = smem + L.offset;
-    const float* rhs = q + L.planes * n1 * n2;
-    for (int idx = threadIdx.x; idx < cells; idx += BOTTOM_THREADS) {
-      L.q[base + idx] = q[idx];
-      if (l > 0) L.rhs[base + idx] = rhs[idx];
-    }
-  }
-  c.cluster.sync();  // no CTA leaves while another may still read its shared memory
-}
-
-// ---- the one-block coarse solve (alternative bottom: every level in one CTA's shared memory) --------------
+// ---- the one-block coarse solve with the coarsest level in double (the defect-correction solve's cycles) ----
 
 struct BlockArgs {
   int count;
@@ -930,7 +660,7 @@ struct BlockArgs {
   PlumeLevel lv[BOTTOM_MAX_LEVELS];
   int offset[BOTTOM_MAX_LEVELS];
   int coef_offset[BOTTOM_MAX_LEVELS];  // a level with overhanging cells: its CellCoef table's float offset (else -1)
-  int f64_offset;  // k_block_solve<true, ...>: the coarsest level's double copy, from this float offset
+  int f64_offset;  // the coarsest level's double copy, from this float offset
 };
 
 // The stencil of one cell of a level with overhanging cells (fill_hi < 1), as neighbor_sum and relaxed compute
@@ -1228,7 +958,7 @@ __device__ __forceinline__ void block_smooth(const PlumeGridInfo& info, float* q
 
 // TABLES: some level has overhanging cells (CellCoef tables in b.coef_offset); without, the uniform levels'
 // code is compiled alone.
-template <bool COARSE_F64, bool TABLES>
+template <bool TABLES>
 __global__ void __launch_bounds__(BOTTOM_THREADS) k_block_solve(BlockArgs b) {
   wait_for_previous_grid();
   extern __shared__ float smem[];
@@ -1298,12 +1028,8 @@ __global__ void __launch_bounds__(BOTTOM_THREADS) k_block_solve(BlockArgs b) {
     const int longest = imax_(d.n0, imax_(d.n1, d.n2));
     const int n = d.n0 * d.n1 * d.n2;
     const int sweeps = imax_(COARSEST_SWEEPS, COARSEST_SWEEPS_PER_CELL * longest);
-    if constexpr (COARSE_F64) {
-      double* staged = reinterpret_cast<double*>(smem + b.f64_offset);
-      coarsest_f64(info, q, q + n, sweeps, 1.5, staged, staged + n);
-    } else {
-      block_smooth(info, q, q + n, sweeps, 1.5f, coef_of(b.count - 1));
-    }
+    double* staged = reinterpret_cast<double*>(smem + b.f64_offset);
+    coarsest_f64(info, q, q + n, sweeps, 1.5, staged, staged + n);
   }
   for (int l = b.count - 2; l >= 0; --l) {
     const PlumeGridInfo& info = b.lv[l].info;
@@ -1510,21 +1236,26 @@ static int sweeps_with_prolong(const PlumeGridInfo& info, Pressure& q, const flo
   return PLUME_OK;
 }
 
+static int prepare_bottom();
+
 // Sweeps on `q` with `scratch` as the second array; the result always ends in `q`.
 int red_black_sweeps(const PlumeGridInfo& info, float* q, float* scratch, const float* rhs, int sweeps,
                      float relaxation, cudaStream_t st) {
+  int status = PLUME_OK;
+  if (g_bottom_kind == 0 && g_bottom_max_cells > 0 && cells_of(info) <= cluster_max_cells(info, true) &&
+      cells_of(info) < g_tiled_min_cells) {  // every sweep in one launch, the level in shared memory
+    if ((status = prepare_bottom()) != PLUME_OK) return status;
+    const PlumeLevel level{info, q, const_cast<float*>(rhs), scratch};
+    const bool single = cells_of(info) <= g_bottom_max_cells && cluster_solve_single(info);
+    const ClusterSolve solve{&level, 1, single ? 0 : 1, single ? 1 : 16, 1, 0, false, false, sweeps, relaxation};
+    if (cluster_solve_runs(solve)) return launch_cluster_solve(solve, pdl_enabled(), st);
+  }
   Pressure p{q, scratch};
-  int status = sweeps_with_prolong(info, p, rhs, sweeps, relaxation, nullptr, nullptr, st);
+  status = sweeps_with_prolong(info, p, rhs, sweeps, relaxation, nullptr, nullptr, st);
   if (status != PLUME_OK || p.cur == q) return status;
   return runtime_status("pressure copy-back", cudaMemcpyAsync(q, p.cur, sizeof(float) * (size_t)cells_of(info),
                                                               cudaMemcpyDeviceToDevice, st));
 }
-
-// The first level from which the rest of the hierarchy runs in one cluster launch (count when none fits),
-// and that launch's per-CTA shared memory.
-// With coarse_f64 the one-block solve is used (it holds the double copy of the coarsest level after the
-// float arrays, 8-byte aligned).
-static int bottom_kind(int coarse_f64) { return coarse_f64 ? 0 : g_bottom_kind; }
 
 static size_t f64_staging_offset(size_t float_bytes) { return (float_bytes + 7) / 8 * 8; }
 
@@ -1545,39 +1276,66 @@ static size_t coef_bytes(const PlumeLevel* levels, int count, size_t bytes, int*
   return bytes;
 }
 
-static int bottom_start(const PlumeLevel* levels, int count, size_t* smem_bytes, int coarse_f64) {
-  for (int first = 0; first < count; ++first) {
-    if (count - first > BOTTOM_MAX_LEVELS || cells_of(levels[first].info) > g_bottom_max_cells) continue;
-    size_t bytes = 0;
-    for (int l = first; l < count; ++l) {
-      const PlumeGridInfo& info = levels[l].info;
-      const bool single = bottom_kind(coarse_f64) == 0 || cells_of(info) <= SINGLE_MAX_CELLS;
-      const long planes = single ? info.dims[0] : (info.dims[0] + CLUSTER - 1) / CLUSTER;
-      bytes += 2 * sizeof(float) * (size_t)planes * info.dims[1] * info.dims[2];
-    }
-    if (bottom_kind(coarse_f64) == 0) bytes = coef_bytes(levels + first, count - first, bytes);
-    if (coarse_f64) bytes = f64_staging_offset(bytes) + 2 * sizeof(double) * (size_t)cells_of(levels[count - 1].info);
-    if (bytes > BOTTOM_MAX_SMEM) continue;
-    *smem_bytes = bytes;
-    return first;
-  }
-  return count;
+// Which levels of a hierarchy run in one launch: from `start` down (count: none), those from `single_from` on in one
+// CTA, with `ctas` CTAs for the levels between, or (coarse_f64) in one block of k_block_solve with `smem` bytes.
+struct CoarsePlan {
+  int start, single_from, ctas;
+  size_t smem;
+  bool store_all = true;  // this cycle is the solve's last: the coarser levels' arrays are left as it has them
+};
+
+static int coarsest_sweeps(const PlumeGridInfo& info) {
+  const int longest = std::max(info.dims[0], std::max(info.dims[1], info.dims[2]));
+  return std::max(COARSEST_SWEEPS, COARSEST_SWEEPS_PER_CELL * longest);
 }
 
-// Lets the coarse solves use up to BOTTOM_MAX_SMEM of shared memory (once per device, outside any capture).
+static ClusterSolve cluster_solve(const PlumeLevel* levels, int count, const CoarsePlan& plan, int cycles, int sweeps,
+                                  bool store_all) {
+  return ClusterSolve{levels + plan.start, count - plan.start, plan.single_from - plan.start, plan.ctas,
+                      cycles, sweeps, plan.start > 0, store_all, coarsest_sweeps(levels[count - 1].info), 1.5f};
+}
+
+// `first_level`: the levels before it are not to be part of the launch.
+static CoarsePlan coarse_plan(const PlumeLevel* levels, int count, int coarse_f64, int first_level) {
+  CoarsePlan plan{count, count, 1, 0};
+  for (int first = first_level; first < count && plan.start == count; ++first) {
+    if (count - first > BOTTOM_MAX_LEVELS || cells_of(levels[first].info) > g_bottom_max_cells) continue;
+    if (coarse_f64) {
+      size_t bytes = 0;
+      for (int l = first; l < count; ++l) bytes += 2 * sizeof(float) * (size_t)cells_of(levels[l].info);
+      bytes = f64_staging_offset(coef_bytes(levels + first, count - first, bytes)) +
+              2 * sizeof(double) * (size_t)cells_of(levels[count - 1].info);
+      if (bytes <= BOTTOM_MAX_SMEM) plan = CoarsePlan{first, first, 1, bytes};
+      continue;
+    }
+    // the first level of one CTA, the rest above it in slabs; then (kind 0) levels above the bottom join the launch
+    const long single_cells = g_bottom_kind == 1 ? std::min(g_bottom_max_cells, SINGLE_MAX_CELLS) : g_bottom_max_cells;
+    int single = first;
+    while (single < count && (cells_of(levels[single].info) > single_cells || !cluster_solve_single(levels[single].info)))
+      ++single;
+    for (int top = g_bottom_kind == 1 ? first : first_level; top <= first && plan.start == count; ++top) {
+      if (top < first && (cells_of(levels[top].info) > cluster_max_cells(levels[top].info, top == 0) || cells_of(levels[top].info) >= g_tiled_min_cells))
+        continue;
+      for (int ctas : {16, 8}) {
+        const CoarsePlan here{top, single, top >= single ? 1 : (g_bottom_kind == 1 ? 8 : ctas), 0};
+        if (plan.start == count && cluster_solve_runs(cluster_solve(levels, count, here, 1, 0, true))) plan = here;
+      }
+    }
+  }
+  return plan;
+}
+
+// Lets the one-launch solves use their shared memory and cluster size (once per device, outside any capture).
 static int prepare_bottom() {
   static std::mutex mutex;
   static bool configured[64] = {};
   int device = 0;
-  int status = runtime_status("current device", cudaGetDevice(&device));
+  int status = prepare_cluster_solve();
   if (status != PLUME_OK) return status;
+  if ((status = runtime_status("current device", cudaGetDevice(&device))) != PLUME_OK) return status;
   std::lock_guard<std::mutex> lock(mutex);
   if (device >= 0 && device < 64 && !configured[device]) {
-    status = runtime_status("coarse solve shared memory",
-                            cudaFuncSetAttribute(k_cluster_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)BOTTOM_MAX_SMEM));
-    for (auto kernel : {k_block_solve<false, false>, k_block_solve<true, false>, k_block_solve<false, true>,
-                        k_block_solve<true, true>})
+    for (auto kernel : {k_block_solve<false>, k_block_solve<true>})
       if (status == PLUME_OK)
         status = runtime_status("coarse solve shared memory",
                                 cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1592,63 +1350,27 @@ static int prepare_bottom() {
   return PLUME_OK;
 }
 
-static int launch_bottom(const PlumeLevel* levels, int count, int sweeps, size_t smem, cudaStream_t st,
-                         int coarse_f64) {
-  int status = prepare_bottom();
-  if (status != PLUME_OK) return status;
-  if (bottom_kind(coarse_f64) == 0) {
-    BlockArgs b{};
-    b.count = count;
-    b.sweeps = sweeps;
-    int offset = 0;
-    for (int l = 0; l < count; ++l) {
-      b.lv[l] = levels[l];
-      b.offset[l] = offset;
-      offset += 2 * (int)cells_of(levels[l].info);
-    }
-    const size_t table_end = coef_bytes(levels, count, sizeof(float) * (size_t)offset, b.coef_offset);
-    b.f64_offset = (int)(f64_staging_offset(table_end) / sizeof(float));
-    bool tables = false;
-    for (int l = 0; l < count; ++l) tables = tables || b.coef_offset[l] >= 0;
-    auto kernel = coarse_f64 ? (tables ? k_block_solve<true, true> : k_block_solve<true, false>)
-                             : (tables ? k_block_solve<false, true> : k_block_solve<false, false>);
-    return launch_solve_kernel(kernel, dim3(1), dim3(BOTTOM_THREADS),
-                               smem, st, "coarse-level block solve", b);
-  }
-  ClusterArgs b{};
+static int launch_block_solve(const PlumeLevel* levels, int count, int sweeps, size_t smem, cudaStream_t st) {
+  BlockArgs b{};
   b.count = count;
   b.sweeps = sweeps;
   int offset = 0;
   for (int l = 0; l < count; ++l) {
-    LevelView& L = b.lv[l];
-    L.info = levels[l].info;
-    L.q = levels[l].q;
-    L.rhs = levels[l].rhs;
-    L.single = cells_of(L.info) <= SINGLE_MAX_CELLS ? 1 : 0;
-    L.planes = L.single ? L.info.dims[0] : (L.info.dims[0] + CLUSTER - 1) / CLUSTER;
-    L.offset = offset;
-    offset += 2 * L.planes * L.info.dims[1] * L.info.dims[2];
+    b.lv[l] = levels[l];
+    b.offset[l] = offset;
+    offset += 2 * (int)cells_of(levels[l].info);
   }
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(CLUSTER, 1, 1);
-  config.blockDim = dim3(BOTTOM_THREADS, 1, 1);
-  config.dynamicSmemBytes = smem;
-  config.stream = st;
-  cudaLaunchAttribute attribute[1];
-  attribute[0].id = cudaLaunchAttributeClusterDimension;
-  attribute[0].val.clusterDim.x = CLUSTER;
-  attribute[0].val.clusterDim.y = 1;
-  attribute[0].val.clusterDim.z = 1;
-  config.attrs = attribute;
-  config.numAttrs = 1;
-  status = runtime_status("coarse-level cluster solve", cudaLaunchKernelEx(&config, k_cluster_solve, b));
-  if (status != PLUME_OK) return status;
-  return launch_status("coarse-level cluster solve");
+  const size_t table_end = coef_bytes(levels, count, sizeof(float) * (size_t)offset, b.coef_offset);
+  b.f64_offset = (int)(f64_staging_offset(table_end) / sizeof(float));
+  bool tables = false;
+  for (int l = 0; l < count; ++l) tables = tables || b.coef_offset[l] >= 0;
+  return launch_solve_kernel(tables ? k_block_solve<true> : k_block_solve<false>, dim3(1), dim3(BOTTOM_THREADS), smem, st,
+                             "coarse-level block solve", b);
 }
 
 // One V-cycle below `index` (multigrid.py:130-147). Every level keeps its pressure in q and uses its residual
 // array as the sweeps' second array; the residual itself is never stored (k_residual_restrict).
-static int v_cycle(const PlumeLevel* levels, int count, int index, Pressure& q, int bottom, size_t smem, int sweeps,
+static int v_cycle(const PlumeLevel* levels, int count, int index, Pressure& q, const CoarsePlan& plan, int sweeps,
                    cudaStream_t st, int coarse_f64, const SplitTop* split = nullptr) {
   const PlumeLevel& lv = levels[index];
   if (index == 0 && split) {  // the top level in split storage (never the bottom or the coarsest level)
@@ -1667,7 +1389,7 @@ static int v_cycle(const PlumeLevel* levels, int count, int index, Pressure& q, 
                                        (const float*)split->rhs, cd, coarse.rhs, coarse.q);
     if (status != PLUME_OK) return status;
     Pressure coarse_q{coarse.q, coarse.residual};
-    if ((status = v_cycle(levels, count, 1, coarse_q, bottom, smem, sweeps, st, coarse_f64)) != PLUME_OK) return status;
+    if ((status = v_cycle(levels, count, 1, coarse_q, plan, sweeps, st, coarse_f64)) != PLUME_OK) return status;
     if (coarse_q.cur != coarse.q) {
       status = runtime_status("coarse pressure copy",
                               cudaMemcpyAsync(coarse.q, coarse_q.cur, sizeof(float) * cd.n0 * cd.n1 * cd.n2,
@@ -1676,24 +1398,20 @@ static int v_cycle(const PlumeLevel* levels, int count, int index, Pressure& q, 
     }
     return split_sweeps(lv.info, *split, sweeps, coarse.q, &coarse.info, st);
   }
-  if (index == bottom) {
-    PlumeLevel first[BOTTOM_MAX_LEVELS];
-    for (int l = bottom; l < count && l - bottom < BOTTOM_MAX_LEVELS; ++l) first[l - bottom] = levels[l];
-    first[0].q = q.cur;
-    return launch_bottom(first, count - bottom, sweeps, smem, st, coarse_f64);
+  if (index == plan.start) {
+    if (coarse_f64) return launch_block_solve(levels + index, count - index, sweeps, plan.smem, st);
+    return launch_cluster_solve(cluster_solve(levels, count, plan, 1, sweeps, plan.store_all), pdl_enabled(), st);
   }
   if (index == count - 1) {
-    const int longest = std::max(lv.info.dims[0], std::max(lv.info.dims[1], lv.info.dims[2]));
     if (coarse_f64) {
       const size_t bytes = 2 * sizeof(double) * (size_t)cells_of(lv.info);
       if (bytes > BOTTOM_MAX_SMEM) return fail(PLUME_ERR_INVALID, "coarsest level too large for the double solve");
       int status = prepare_bottom();
       if (status != PLUME_OK) return status;
       return launch_solve_kernel(k_coarsest_f64, dim3(1), dim3(BOTTOM_THREADS), bytes, st, "coarsest double solve",
-                                 lv.info, q.cur, lv.rhs, std::max(COARSEST_SWEEPS, COARSEST_SWEEPS_PER_CELL * longest));
+                                 lv.info, q.cur, lv.rhs, coarsest_sweeps(lv.info));
     }
-    return sweeps_with_prolong(lv.info, q, lv.rhs, std::max(COARSEST_SWEEPS, COARSEST_SWEEPS_PER_CELL * longest), 1.5f,
-                               nullptr, nullptr, st);
+    return sweeps_with_prolong(lv.info, q, lv.rhs, coarsest_sweeps(lv.info), 1.5f, nullptr, nullptr, st);
   }
   int status = sweeps_with_prolong(lv.info, q, lv.rhs, sweeps, 1.0f, nullptr, nullptr, st);
   if (status != PLUME_OK) return status;
@@ -1704,7 +1422,7 @@ static int v_cycle(const PlumeLevel* levels, int count, int index, Pressure& q, 
       PLUME_OK)
     return status;
   Pressure coarse_q{coarse.q, coarse.residual};
-  if ((status = v_cycle(levels, count, index + 1, coarse_q, bottom, smem, sweeps, st, coarse_f64)) != PLUME_OK)
+  if ((status = v_cycle(levels, count, index + 1, coarse_q, plan, sweeps, st, coarse_f64)) != PLUME_OK)
     return status;
   if (coarse_q.cur != coarse.q) {  // an odd number of coarsest sweeps left the result in the second array
     status = runtime_status("coarse pressure copy", cudaMemcpyAsync(coarse.q, coarse_q.cur, sizeof(float) * cd.n0 * cd.n1 * cd.n2,
@@ -1714,19 +1432,20 @@ static int v_cycle(const PlumeLevel* levels, int count, int index, Pressure& q, 
   return sweeps_with_prolong(lv.info, q, lv.rhs, sweeps, 1.0f, coarse.q, &coarse.info, st);
 }
 
-// Whether the top level runs split: scratch given, at least two levels with level 0 above the bottom solve,
-// uniform couplings, swept by colour (not tiled) and at least g_split_min_cells cells.
-static bool use_split(const PlumeLevel* levels, int count, int bottom, const float* scratch) {
+// Whether the top level runs split: scratch given, at least two levels with level 0 above the bottom (a level of
+// at most g_bottom_max_cells), uniform couplings, swept by colour (not tiled) and at least g_split_min_cells cells.
+static bool use_split(const PlumeLevel* levels, int count, int coarse_f64, const float* scratch) {
   const PlumeGridInfo& info = levels[0].info;
-  return scratch && ((uintptr_t)scratch & 15) == 0 && count >= 2 && bottom > 0 && uniform_level(info) &&
-         cells_of(info) >= g_split_min_cells && cells_of(info) < g_tiled_min_cells;
+  return scratch && ((uintptr_t)scratch & 15) == 0 && count >= 2 && uniform_level(info) &&
+         cells_of(info) >= g_split_min_cells && cells_of(info) < g_tiled_min_cells &&
+         coarse_plan(levels, count, coarse_f64, 0).single_from > 0;
 }
 
 static int multigrid_direct(const PlumeLevel* levels, int count, int cycles, int sweeps, cudaStream_t st,
                             int coarse_f64, float* split_scratch = nullptr) {
-  size_t smem = 0;
-  const int bottom = bottom_start(levels, count, &smem, coarse_f64);
-  if (use_split(levels, count, bottom, split_scratch)) {
+  const bool split = use_split(levels, count, coarse_f64, split_scratch);
+  CoarsePlan plan = coarse_plan(levels, count, coarse_f64, split ? 1 : 0);
+  if (split) {
     const PlumeGridInfo& info = levels[0].info;
     const Dims d = dims_of(info);
     SplitTop sp{split_scratch, split_scratch + split_floats(info), split_H(info)};
@@ -1738,15 +1457,20 @@ static int multigrid_direct(const PlumeLevel* levels, int count, int cycles, int
                                       d, sp.H, (const float*)levels[0].rhs, sp.rhs)) != PLUME_OK)
       return status;
     Pressure unused{levels[0].q, levels[0].residual};
-    for (int c = 0; c < cycles; ++c)
-      if ((status = v_cycle(levels, count, 0, unused, bottom, smem, sweeps, st, coarse_f64, &sp)) != PLUME_OK)
+    for (int c = 0; c < cycles; ++c) {
+      plan.store_all = c == cycles - 1;
+      if ((status = v_cycle(levels, count, 0, unused, plan, sweeps, st, coarse_f64, &sp)) != PLUME_OK)
         return status;
+    }
     return launch_solve_kernel(k_split_layout<false>, grid, cell_block(), 0, st, "pressure from split storage", d,
                                sp.H, (const float*)sp.q, levels[0].q);
   }
+  if (plan.start == 0 && !coarse_f64 && cycles > 0)
+    return launch_cluster_solve(cluster_solve(levels, count, plan, cycles, sweeps, true), pdl_enabled(), st);
   Pressure q{levels[0].q, levels[0].residual};
   for (int c = 0; c < cycles; ++c) {
-    int status = v_cycle(levels, count, 0, q, bottom, smem, sweeps, st, coarse_f64);
+    plan.store_all = c == cycles - 1;
+    int status = v_cycle(levels, count, 0, q, plan, sweeps, st, coarse_f64);
     if (status != PLUME_OK) return status;
   }
   if (q.cur == levels[0].q) return PLUME_OK;
@@ -1843,6 +1567,8 @@ int multigrid_cycles(const PlumeLevel* levels, int count, int cycles, int sweeps
                      float* split_scratch) {
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   int device = 0;
+  int prepared = prepare_bottom();
+  if (prepared != PLUME_OK) return prepared;
   if (!g_use_graphs || count > 16 || cudaStreamIsCapturing(st, &capturing) != cudaSuccess ||
       capturing != cudaStreamCaptureStatusNone || cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64)
     return multigrid_direct(levels, count, cycles, sweeps, st, coarse_f64, split_scratch);
@@ -1860,13 +1586,6 @@ int multigrid_cycles(const PlumeLevel* levels, int count, int cycles, int sweeps
   key.split = split_scratch;
   std::memcpy(key.levels, levels, sizeof(PlumeLevel) * count);
   std::lock_guard<std::mutex> lock(g_graph_mutex);
-  {  // the coarse solve's shared-memory attribute must be set before its first capture
-    size_t smem = 0;
-    if (bottom_start(levels, count, &smem, coarse_f64) < count || coarse_f64) {
-      int prepared = prepare_bottom();
-      if (prepared != PLUME_OK) return prepared;
-    }
-  }
   cudaGraphExec_t exec = nullptr;
   size_t kernels = 0;
   int status = graph_for(key, levels, &exec, &kernels);

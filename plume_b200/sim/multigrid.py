@@ -25,8 +25,8 @@ SMOOTHING_RELAXATION = 1.0
 class SolverTuning:
     """The library's pressure-solve strategy (results do not depend on it): levels of at least
     `tiled_min_cells` cells sweep in shared-memory tiles, one launch per sweep; smaller ones one colour per
-    launch; the first level of at most `bottom_max_cells` cells and all coarser ones run in one launch
-    (`bottom_kind` 0 one block, 1 an 8-CTA cluster)."""
+    launch; the first level of at most `bottom_max_cells` cells and all coarser ones run in one launch of one
+    thread-block cluster (`bottom_kind` 0: 16 CTAs, larger levels above the bottom in the same launch; 1: 8 CTAs)."""
 
     tiled_min_cells: int
     bottom_max_cells: int
