@@ -26,17 +26,15 @@
 // only. Halo planes outside the level and the padding slot of an odd row hold 0, which is what neighbor_sum adds
 // for a missing neighbour. Levels from `single_from` on sit in CTA 0 in natural layout.
 //
-// Stencils. A cell's couplings depend on its position along each axis only through four classes (first cell,
-// interior, last but one, last: fill_hi and the faces enter nowhere else), so each level has a table of 64
-// stencils, built once per launch with the reference's operations. The quotient (sq - source) / sc is the product
-// with the table's double reciprocal of sc (quotient() below), which is the IEEE quotient.
+// Stencils come from a table per level by cell class (stencil_table.cuh), built once per launch with the reference's
+// operations. The quotient (sq - source) / sc is the product with the table's double reciprocal of sc.
 #include <cooperative_groups.h>
 
 #include <algorithm>
 #include <mutex>
 
 #include "cluster_solve.cuh"
-#include "poisson.cuh"
+#include "stencil_table.cuh"
 
 namespace plume {
 
@@ -45,14 +43,6 @@ namespace cg = cooperative_groups;
 constexpr int CS_THREADS = 512;
 constexpr size_t CS_MAX_SMEM = 220 * 1024;
 
-// The stencil of one class of cells: neighbor_sum's couplings (x-, x+, y-, y+, z-, z+; a ghost's coupling, or 0
-// for a closed face, where the neighbour is outside the level), their sum, cell_volume * cell_m * cell_m, and the
-// reciprocals of those two in double.
-struct __align__(16) ClassStencil {
-  float c[6];
-  float sc, vc;
-  double inv, inv_vc;
-};
 constexpr int STENCIL_FLOATS = sizeof(ClassStencil) / sizeof(float);
 
 // x / d and x % d for 0 <= x < 65536, d < 65536 by one multiplication: inverse = ceil(2^32 / d), 0 for d = 1.
@@ -85,24 +75,6 @@ struct ClusterArgs {
 };
 
 extern __shared__ __align__(16) float smem[];
-
-__device__ __forceinline__ int class_of(int index, int n) {
-  return index == n - 1 ? 3 : (index == n - 2 ? 2 : (index == 0 ? 0 : 1));
-}
-__device__ __forceinline__ int class_index(int cls, int n) {  // a cell index of the class (any, when it has none)
-  return cls == 3 ? n - 1 : (cls == 2 ? imax_(n - 2, 0) : (cls == 0 ? 0 : imin_(1, n - 1)));
-}
-
-// x / d, correctly rounded, as the product with a double within 2^-52 (relative) of 1 / d. The product is then within
-// 2^-51 of x / d. A quotient of two floats never is the midpoint m of two neighbouring normal
-// floats, and x - m d, a multiple of the last place of the 49-bit product m d, then differs from 0 by at least
-// 2^-49 of x: so the product and x / d round to the same float. (The range of a double holds every case: zeros,
-// infinities and NaN come out as the division's too.) Unlike the division, and unlike a float reciprocal with
-// remainder steps, this has no branch for operands out of range: in these passes, which a few warps run once
-// through, a branch over a slow path costs more than the arithmetic, since the instructions after it are fetched
-// late. Measured on B200, one dependent update on one warp: 115 cycles, with float remainder steps behind a range
-// test 350 (118 only as a loop of that body alone).
-__device__ __forceinline__ float quotient(float x, double inv) { return (float)((double)x * inv); }
 
 // 1 / d for quotient(): two Newton steps in double from the approximate float reciprocal (relative error 2^-23, then
 // 2^-46, then the double's rounding), without a division's branch.

@@ -21,7 +21,7 @@
 #include <vector>
 
 #include "cluster_solve.cuh"
-#include "poisson.cuh"
+#include "stencil_table.cuh"
 
 namespace plume {
 
@@ -141,96 +141,235 @@ __global__ void __launch_bounds__(SWEEP_THREADS)
   }
 }
 
-// One colour of a sweep in place (red_black_sweep_kernel, pressure.py:80-92): for levels too small to fill
-// the GPU with tiles. A colour reads only the other colour, so the in-place update is race-free.
+// ---- levels swept by colour in the natural layout ----------------------------------------------------------------
+// One colour of a sweep in place (red_black_sweep_kernel, pressure.py:80-92). A colour reads only the other colour, so
+// the in-place update is race-free. The kernels below have no branch over code that does not run: a missing
+// neighbour's load goes to the cell's own row and its value is replaced by the 0 that neighbor_sum adds, couplings come
+// from the level's class table, quotients are products with double reciprocals.
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+
+__device__ __forceinline__ float coupled_sum(const ClassStencil& e, float xm, float xp, float ym, float yp, float zm, float zp) {
+  return ((((e.c[0] * xm + e.c[1] * xp) + e.c[2] * ym) + e.c[3] * yp) + e.c[4] * zm) + e.c[5] * zp;
+}
+__device__ __forceinline__ float plain_sum(float xm, float xp, float ym, float yp, float zm, float zp) {
+  return ((((xm + xp) + ym) + yp) + zm) + zp;
+}
+
+// One cell per thread, rows of any length.
 template <bool UNIFORM>
-__global__ void k_rb_colour(PlumeGridInfo info, float* q, const float* __restrict__ rhs, int color, float relaxation,
-                            const float* __restrict__ coarse_q, Dims coarse) {
+__global__ void k_colour_cells(const __grid_constant__ LevelTable t, Dims d, float* q, const float* __restrict__ rhs,
+                               int color, float relaxation) {
   wait_for_previous_grid();
-  const int ny = info.dims[1], nz = info.dims[2];
   const int i = blockIdx.z, j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + ((i + j + color) & 1);
-  if (j >= ny || k >= nz) return;
-  const Dims d = dims_of(info);
-  auto load = [&](int a, int b, int c) { return q[at(d, a, b, c)]; };
-  const int idx = at(d, i, j, k);
-  float out;
-  if (relax_cell(UNIFORM, info, ghost_coupling(info), i, j, k, q[idx], __ldg(rhs + idx), relaxation, load, out))
-    q[idx] = out;
+  if (j >= d.n1 || k >= d.n2) return;
+  const int plane = d.n1 * d.n2, at_c = at(d, i, j, k);
+  const bool x0 = i > 0, x1 = i < d.n0 - 1, y0 = j > 0, y1 = j < d.n1 - 1, z0 = k > 0, z1 = k < d.n2 - 1;
+  const float vxm = q[x0 ? at_c - plane : at_c], vxp = q[x1 ? at_c + plane : at_c];
+  const float vym = q[y0 ? at_c - d.n2 : at_c], vyp = q[y1 ? at_c + d.n2 : at_c];
+  const float vzm = q[z0 ? at_c - 1 : at_c], vzp = q[z1 ? at_c + 1 : at_c];
+  const float xm = x0 ? vxm : 0.0f, xp = x1 ? vxp : 0.0f, ym = y0 ? vym : 0.0f, yp = y1 ? vyp : 0.0f;
+  const float zm = z0 ? vzm : 0.0f, zp = z1 ? vzp : 0.0f;
+  const float own = q[at_c], r = __ldg(rhs + at_c);
+  const ClassStencil& e = t.e[16 * class_of(i, d.n0) + 4 * class_of(j, d.n1) + class_of(k, d.n2)];
+  const float sq = UNIFORM ? plain_sum(xm, xp, ym, yp, zm, zp) : coupled_sum(e, xm, xp, ym, yp, zm, zp);
+  const float value = own + relaxation * (quotient(sq - e.vc * r, e.inv) - own);
+  q[at_c] = UNIFORM || e.sc != 0.0f ? value : own;  // a cell with no coupling at all (a level of one cell) is left alone
 }
 
-// The same colour pass with each thread updating one cell in each of two neighbouring planes (i, i + 1): two
-// independent updates whose loads are in flight together. The two cells are the same colour and not face
-// neighbours, and every update is the one above, so the result is the same. Measured on B200: the 4-cycle
-// solve at 256x384x256 went from 3.727 to 3.570 ms with every level swept this way, but at 128x192x128 from
-// 0.780 to 0.828 ms: it pays only on levels that do not fit in L2 (RB_PAIR_MIN_CELLS).
+// Four consecutive cells of a row per thread, two of them of the colour: 16-byte loads of the row, of its four
+// neighbouring rows and of rhs, and the one value beyond the four that the row's parity needs. The other colour's two
+// values are stored back unchanged: this pass never writes them, so any thread reading them sees the same floats. Rows
+// of a multiple of four cells, 16-byte-aligned arrays. Measured on B200 at 128x192x128, one pass cold: 7.8 us; with the
+// row-interior and boundary cases as branches and the division by six behind a range test 9.9 us.
 template <bool UNIFORM>
-__global__ void k_rb_colour_pair(PlumeGridInfo info, float* q, const float* __restrict__ rhs, int color,
-                                 float relaxation) {
+__global__ void k_colour_rows4(const __grid_constant__ LevelTable t, Dims d, float* __restrict__ q,
+                               const float* __restrict__ rhs, int color, float relaxation) {
   wait_for_previous_grid();
-  const int nx = info.dims[0], ny = info.dims[1], nz = info.dims[2];
-  const int i = 2 * blockIdx.z, j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int kp = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
-  const int k0 = kp + ((i + j + color) & 1), k1 = kp + ((i + 1 + j + color) & 1);
-  if (j >= ny) return;
-  const bool has0 = k0 < nz, has1 = i + 1 < nx && k1 < nz;
-  const Dims d = dims_of(info);
-  auto load = [&](int a, int b, int c) { return q[at(d, a, b, c)]; };
-  const float ghost = ghost_coupling(info);
-  const int idx0 = at(d, i, j, k0), idx1 = at(d, i + 1, j, k1);
-  float out0 = 0.0f, out1 = 0.0f;
-  bool w0 = false, w1 = false;
-  if (has0) w0 = relax_cell(UNIFORM, info, ghost, i, j, k0, q[idx0], __ldg(rhs + idx0), relaxation, load, out0);
-  if (has1) w1 = relax_cell(UNIFORM, info, ghost, i + 1, j, k1, q[idx1], __ldg(rhs + idx1), relaxation, load, out1);
-  if (w0) q[idx0] = out0;
-  if (w1) q[idx1] = out1;
+  const int i = blockIdx.z, j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int k0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (j >= d.n1 || k0 >= d.n2) return;
+  const bool odd = (i + j + color) & 1;  // this colour's cells: k0 + odd and k0 + odd + 2
+  const int plane = d.n1 * d.n2, row = (i * d.n1 + j) * d.n2 + k0;
+  const bool x0 = i > 0, x1 = i < d.n0 - 1, y0 = j > 0, y1 = j < d.n1 - 1;
+  const float4 c = ld4(q + row), r = ldg4(rhs + row);
+  const float4 xm = ld4(q + (x0 ? row - plane : row)), xp = ld4(q + (x1 ? row + plane : row));
+  const float4 ym = ld4(q + (y0 ? row - d.n2 : row)), yp = ld4(q + (y1 ? row + d.n2 : row));
+  const int beyond = odd ? k0 + 4 : k0 - 1;
+  const bool has_far = beyond >= 0 && beyond < d.n2;
+  const float far_value = q[row + (has_far ? beyond - k0 : 0)], far = has_far ? far_value : 0.0f;
+  auto pick = [&](const float4& v, int n) { return n == 0 ? (odd ? v.y : v.x) : (odd ? v.w : v.z); };
+  const float o0 = odd ? c.x : c.y, o1 = odd ? c.z : c.w;  // the other colour's two
+  const ClassStencil* table = t.e + 16 * class_of(i, d.n0) + 4 * class_of(j, d.n1);
+  float out[2];
+#pragma unroll
+  for (int n = 0; n < 2; ++n) {
+    const int k = k0 + (odd ? 1 : 0) + 2 * n;
+    const float a = x0 ? pick(xm, n) : 0.0f, b = x1 ? pick(xp, n) : 0.0f;
+    const float e0 = y0 ? pick(ym, n) : 0.0f, e1 = y1 ? pick(yp, n) : 0.0f;
+    const float zm = n == 0 ? (odd ? o0 : far) : (odd ? o1 : o0), zp = n == 0 ? (odd ? o1 : o0) : (odd ? far : o1);
+    const ClassStencil& e = table[class_of(k, d.n2)];
+    const float sq = UNIFORM ? plain_sum(a, b, e0, e1, zm, zp) : coupled_sum(e, a, b, e0, e1, zm, zp);
+    const float own = pick(c, n);
+    out[n] = own + relaxation * (quotient(sq - e.vc * pick(r, n), e.inv) - own);
+  }
+  *reinterpret_cast<float4*>(q + row) = odd ? make_float4(c.x, out[0], c.z, out[1]) : make_float4(out[0], c.y, out[1], c.w);
 }
 
-// prolong_add_kernel (multigrid.py:63-68), used when a level has no post-smoothing sweep to fold it into.
-__global__ void k_prolong_add(Dims coarse, Dims fine, const float* __restrict__ cq, float* __restrict__ q) {
-  wait_for_previous_grid();
-  const int i = blockIdx.z, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= fine.n1 || k >= fine.n2) return;
-  const int idx = at(fine, i, j, k);
-  q[idx] = q[idx] + sample_index_space(cq, coarse, prolong_point(i, j, k));
+// Four consecutive cells k0 .. k0 + 3 of a row (p: the cell k0): one 16-byte load where rows hold a multiple of four
+// cells and arrays are aligned (WIDE), else four 4-byte loads, with 0 beyond the row's end.
+struct Quad {
+  float v[4];
+  __device__ __forceinline__ Quad() {}
+  __device__ __forceinline__ Quad(float4 a) : v{a.x, a.y, a.z, a.w} {}
+};
+
+template <bool WIDE>
+__device__ __forceinline__ Quad load_quad(const float* p, int k0, int n2) {
+  if constexpr (WIDE) return Quad(ldg4(p));
+  Quad r;
+#pragma unroll
+  for (int n = 0; n < 4; ++n) {
+    const bool there = k0 + n < n2;
+    const float value = __ldg(p + (there ? n : 0));
+    r.v[n] = there ? value : 0.0f;
+  }
+  return r;
 }
 
-// residual_kernel + restrict_kernel (multigrid.py:36-60) + coarse.q.zero_() (:143): each coarse cell averages
-// the residuals of its (up to 8) children, summed in the reference's child order.
-__global__ void k_residual_restrict(PlumeGridInfo fine, const float* __restrict__ q, const float* __restrict__ rhs,
-                                    Dims coarse, float* __restrict__ coarse_rhs, float* __restrict__ coarse_q) {
+__device__ __forceinline__ Quad where(bool there, const Quad& a) {
+  Quad r;
+#pragma unroll
+  for (int n = 0; n < 4; ++n) r.v[n] = there ? a.v[n] : 0.0f;
+  return r;
+}
+
+// prolong_add_kernel (multigrid.py:63-68), four consecutive cells k0 .. k0 + 3 of a row per thread: they
+// share the coarse sample's x and y axes, and along z they read the coarse columns m - 1 .. m + 2 (m = k0 / 2, clamped),
+// each blended in x then y once. Cell k0 + n sits at coarse z = m - 0.25, m + 0.25, m + 0.75, m + 1.25: exact weights,
+// except where the clamp gives the first or the last column the weight 1 (k = 0, and k = n2 - 1 of an even n2). Every
+// operation is sample_index_space's. Measured on B200 at 128x192x128, cold: 8.3 us against 16.2 us with one cell per
+// thread.
+template <bool WIDE>
+__global__ void k_prolong_rows4(Dims coarse, Dims fine, const float* __restrict__ cq, float* __restrict__ q) {
   wait_for_previous_grid();
-  const int i = blockIdx.z, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= coarse.n1 || k >= coarse.n2) return;
-  const Dims fd = dims_of(fine);
-  auto load = [&](int a, int b, int c) { return __ldg(q + at(fd, a, b, c)); };
-  const bool uniform = is_uniform(fine);
-  const float ghost = ghost_coupling(fine);
-  float total = 0.0f, count = 0.0f;
+  const int i = blockIdx.z, j = blockIdx.y * blockDim.y + threadIdx.y, k0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (j >= fine.n1 || k0 >= fine.n2) return;
+  const F3 g = prolong_point(i, j, 0);
+  const Axis1 x = axis_of(g[0], coarse.n0, coarse.n1 * coarse.n2), y = axis_of(g[1], coarse.n1, coarse.n2);
+  const int m = k0 / 2, end = coarse.n2 - 1 - m;  // the last column, from column m
+  const float* base = cq + (x.i0 * coarse.n1 + y.i0) * coarse.n2 + m;
+  const float* rows[4] = {base, base + x.step, base + y.step, base + x.step + y.step};
+  float* const row = q + at(fine, i, j, k0);
+  Quad own;
+  if constexpr (WIDE) {
+    own = Quad(ld4(row));
+  } else {
+#pragma unroll
+    for (int n = 0; n < 4; ++n) own.v[n] = row[k0 + n < fine.n2 ? n : 0];
+  }
+  float c[4][4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    c[r][0] = __ldg(rows[r] + (k0 == 0 ? 0 : -1));
+    if constexpr (WIDE) {
+      const float2 mid = __ldg(reinterpret_cast<const float2*>(rows[r]));
+      c[r][1] = mid.x;
+      c[r][2] = mid.y;
+    } else {
+      c[r][1] = __ldg(rows[r]);
+      c[r][2] = __ldg(rows[r] + imin_(1, end));
+    }
+    c[r][3] = __ldg(rows[r] + imin_(2, end));
+  }
+  float e[4];
+#pragma unroll
+  for (int o = 0; o < 4; ++o) e[o] = lerp_w(lerp_w(c[0][o], c[1][o], x), lerp_w(c[2][o], c[3][o], x), y);
+  const bool front = k0 == 0;
+#pragma unroll
+  for (int n = 0; n < 4; ++n) {
+    // columns (n + 1) / 2 and (n + 1) / 2 + 1 of e, weights 0.25 and 0.75 or 0.75 and 0.25; at a clamp the first two
+    // columns, or the last one twice, with weights 1 and 0
+    const int lo = (n + 1) / 2;
+    const bool first = n == 0 && front, last = (n & 1) && m + n / 2 >= coarse.n2 - 1, clamped = first || last;
+    const float a = first ? e[1] : e[lo], b = first ? e[2] : (last ? e[lo] : e[lo + 1]);
+    own.v[n] = own.v[n] + (a * (clamped ? 1.0f : (n & 1 ? 0.75f : 0.25f)) + b * (clamped ? 0.0f : (n & 1 ? 0.25f : 0.75f)));
+  }
+  if constexpr (WIDE) {
+    *reinterpret_cast<float4*>(row) = make_float4(own.v[0], own.v[1], own.v[2], own.v[3]);
+  } else {
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+      if (k0 + n < fine.n2) row[n] = own.v[n];
+  }
+}
+
+// residual_kernel + restrict_kernel (multigrid.py:36-60) + coarse.q.zero_() (:143): each coarse cell averages the
+// residuals of its (up to 8) children, summed in the reference's child order. Two coarse cells per thread: the children
+// are four consecutive cells k0 .. k0 + 3 of two rows in two planes, loaded as rows with the eight rows around them.
+// Measured on B200 at 128x192x128, cold: 10.0 us against 17.7 us with one coarse cell per thread.
+template <bool UNIFORM, bool WIDE>
+__global__ void k_residual_restrict(const __grid_constant__ LevelTable t, Dims fd, const float* __restrict__ q,
+                                    const float* __restrict__ rhs, Dims coarse, float* __restrict__ coarse_rhs,
+                                    float* __restrict__ coarse_q) {
+  wait_for_previous_grid();
+  const int i = blockIdx.z, j = blockIdx.y * blockDim.y + threadIdx.y, k0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (j >= coarse.n1 || k0 >= fd.n2) return;
+  const int plane = fd.n1 * fd.n2;
+  const bool two_i = 2 * i + 1 < fd.n0, two_j = 2 * j + 1 < fd.n1, front = k0 == 0, back = k0 + 4 >= fd.n2;
+  const int corner = at(fd, 2 * i, 2 * j, k0);
+  int row[2][2];
+  Quad own[2][2];
 #pragma unroll
   for (int di = 0; di < 2; ++di)
 #pragma unroll
-    for (int dj = 0; dj < 2; ++dj)
+    for (int dj = 0; dj < 2; ++dj) {  // a missing child row: the first one's, its value never used
+      row[di][dj] = corner + (di && two_i ? plane : 0) + (dj && two_j ? fd.n2 : 0);
+      own[di][dj] = load_quad<WIDE>(q + row[di][dj], k0, fd.n2);
+    }
+  float total[2] = {0.0f, 0.0f};
 #pragma unroll
-      for (int dk = 0; dk < 2; ++dk) {
-        const int fi = 2 * i + di, fj = 2 * j + dj, fk = 2 * k + dk;
-        if (fi < fd.n0 && fj < fd.n1 && fk < fd.n2) {
-          const int idx = at(fd, fi, fj, fk);
-          if (uniform && fi > 0 && fi < fd.n0 - 1 && fj > 0 && fj < fd.n1 - 1) {
-            const int plane = fd.n1 * fd.n2;
-            const float zm = fk > 0 ? __ldg(q + idx - 1) : 0.0f, zp = fk < fd.n2 - 1 ? __ldg(q + idx + 1) : 0.0f;
-            total = total + residual_xy_interior(fine, ghost, fk, __ldg(q + idx), __ldg(rhs + idx), __ldg(q + idx - plane),
-                                                 __ldg(q + idx + plane), __ldg(q + idx - fd.n2), __ldg(q + idx + fd.n2),
-                                                 zm, zp);
-          } else {
-            total = total + residual_cell(uniform, fine, ghost, fi, fj, fk, __ldg(q + idx), __ldg(rhs + idx), load);
-          }
-          count = count + 1.0f;
-        }
+  for (int di = 0; di < 2; ++di)
+#pragma unroll
+    for (int dj = 0; dj < 2; ++dj) {
+      const int fi = 2 * i + di, fj = 2 * j + dj, c = row[di][dj];
+      const bool there = (di == 0 || two_i) && (dj == 0 || two_j);
+      const bool x0 = fi > 0, x1 = fi < fd.n0 - 1, y0 = fj > 0, y1 = fj < fd.n1 - 1;
+      const bool x_out = di == 0 ? x0 : x1, y_out = dj == 0 ? y0 : y1;  // the rows beyond the children's
+      const int x_step = di == 0 ? -plane : plane, y_step = dj == 0 ? -fd.n2 : fd.n2;
+      const Quad x_row = where(x_out, load_quad<WIDE>(q + (x_out ? c + x_step : c), k0, fd.n2));
+      const Quad y_row = where(y_out, load_quad<WIDE>(q + (y_out ? c + y_step : c), k0, fd.n2));
+      const Quad xm = di == 0 ? x_row : own[0][dj], xp = di == 0 ? where(x1, own[1][dj]) : x_row;
+      const Quad ym = dj == 0 ? y_row : own[di][0], yp = dj == 0 ? where(y1, own[di][1]) : y_row;
+      const float vl = __ldg(q + c + (front ? 0 : -1)), vr = __ldg(q + c + (back ? 0 : 4));
+      const float left = front ? 0.0f : vl, right = back ? 0.0f : vr;
+      const Quad r = load_quad<WIDE>(rhs + c, k0, fd.n2);
+      const ClassStencil* table = t.e + 16 * class_of(imin_(fi, fd.n0 - 1), fd.n0) + 4 * class_of(imin_(fj, fd.n1 - 1), fd.n1);
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const float* o = own[di][dj].v;
+        const float zm = n == 0 ? left : o[n > 0 ? n - 1 : 0], zp = n == 3 ? right : o[n < 3 ? n + 1 : 3];
+        const ClassStencil& e = table[class_of(k0 + n, fd.n2)];
+        const float sq = UNIFORM ? plain_sum(xm.v[n], xp.v[n], ym.v[n], yp.v[n], zm, zp)
+                                 : coupled_sum(e, xm.v[n], xp.v[n], ym.v[n], yp.v[n], zm, zp);
+        const float sum = total[n / 2] + (r.v[n] - quotient(sq - e.sc * o[n], e.inv_vc));
+        total[n / 2] = there && (WIDE || k0 + n < fd.n2) ? sum : total[n / 2];
       }
-  const int out = at(coarse, i, j, k);
-  coarse_rhs[out] = divide(total, divisor(count));  // count is 1, 2, 4 or 8
-  coarse_q[out] = 0.0f;
+    }
+  const float share = (two_i ? 0.5f : 1.0f) * (two_j ? 0.5f : 1.0f);
+  const int out = at(coarse, i, j, k0 / 2);
+  if constexpr (WIDE) {
+    *reinterpret_cast<float2*>(coarse_rhs + out) = make_float2(total[0] * (0.5f * share), total[1] * (0.5f * share));
+    *reinterpret_cast<float2*>(coarse_q + out) = make_float2(0.0f, 0.0f);
+  } else {
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      if (k0 / 2 + n >= coarse.n2) break;
+      coarse_rhs[out + n] = total[n] * (k0 + 2 * n + 1 < fd.n2 ? 0.5f * share : share);  // / 1, 2, 4 or 8: the same float
+      coarse_q[out + n] = 0.0f;
+    }
+  }
 }
 
 // ---- the top level in colour-split storage -----------------------------------------------------------------
@@ -262,277 +401,144 @@ __global__ void k_split_layout(Dims d, int H, const float* __restrict__ in, floa
   }
 }
 
-// The same colour pass with four cells of a row per thread and 16-byte loads: the thread's own q and rhs, the
-// other colour's rows one plane and one row away (x and y neighbours, at the same half indices), and the other
-// colour's own row (z neighbours) plus the one value beyond the four that the row's parity needs. Rows are
-// padded to a multiple of four. Every cell's update is relax_cell's, its neighbours taken from those values.
-__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
-
-// The cells of a row with all four x and y neighbours (the row is neither on a face of the level in x or y):
-// relaxed_uniform's floats with straight-line arithmetic. A z neighbour beyond the level reads 0 (the value
-// beyond the row, and the split rows' padding slots, hold 0), which is what neighbor_sum_uniform adds there; the
-// two cells at the row's ends divide by its couplings, every other cell by six (div6's reciprocal form, with
-// IEEE division where x is outside its range).
-template <int P>
-__device__ __forceinline__ void split_row_interior(const PlumeGridInfo& info, int H, float* __restrict__ qs,
-                                                   const float* __restrict__ rs, long own, long oth, long plane,
-                                                   int m0, float relaxation) {
-  const int nz = info.dims[2];
+// One colour pass with four cells of a row per thread and 16-byte loads: the thread's own q and rhs, the other colour's
+// rows one plane and one row away (x and y neighbours, at the same half indices), and the other colour's own row (z
+// neighbours) plus the one value beyond the four that the row's parity needs. Rows are padded to a multiple of four; a
+// padding slot stays 0, which is also what a missing z neighbour adds. Uniform levels. Measured on B200 at 256x384x256,
+// one pass cold: 34.7 us; with separate row-interior and boundary code and the division by six behind a range test
+// 36.8 us. Its 176 MB take 27 us at the copy rate.
+__global__ void k_rb_split4(const __grid_constant__ LevelTable t, Dims d, int H, float* __restrict__ qs,
+                            const float* __restrict__ rs, int color, float relaxation) {
+  wait_for_previous_grid();
+  const int i = blockIdx.z, j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int m0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (j >= d.n1 || m0 >= H) return;
+  const bool odd = (i + j + color) & 1;  // cell k = 2 m + odd
+  const long plane = (long)d.n1 * H;
+  const long own = ((long)(color * d.n0 + i) * d.n1 + j) * H + m0;
+  const long oth = ((long)((1 - color) * d.n0 + i) * d.n1 + j) * H + m0;  // not written by this pass
+  const bool x0 = i > 0, x1 = i < d.n0 - 1, y0 = j > 0, y1 = j < d.n1 - 1;
   const float4 q4 = ld4(qs + own), r4 = ldg4(rs + own);
-  const float4 x0 = ldg4(qs + oth - plane), x1 = ldg4(qs + oth + plane);
-  const float4 y0 = ldg4(qs + oth - H), y1 = ldg4(qs + oth + H);
+  const float4 xm = ldg4(qs + (x0 ? oth - plane : oth)), xp = ldg4(qs + (x1 ? oth + plane : oth));
+  const float4 ym = ldg4(qs + (y0 ? oth - H : oth)), yp = ldg4(qs + (y1 ? oth + H : oth));
   const float4 zc = ldg4(qs + oth);
-  const int mz = P == 0 ? m0 - 1 : m0 + 4;  // the other colour's value beyond the four that this parity needs
-  const float zx = (P == 0 ? mz >= 0 : mz < H) ? __ldg(qs + oth - m0 + mz) : 0.0f;
-  const float zs[6] = {P == 0 ? zx : 0.0f, zc.x, zc.y, zc.z, zc.w, P == 0 ? 0.0f : zx};  // m0 - 1 .. m0 + 4
+  const bool has_far = odd ? m0 + 4 < H : m0 > 0;
+  const float far_value = __ldg(qs + oth + (has_far ? (odd ? 4 : -1) : 0)), far = has_far ? far_value : 0.0f;
   const float qv[4] = {q4.x, q4.y, q4.z, q4.w}, rv[4] = {r4.x, r4.y, r4.z, r4.w};
-  const float xa[4] = {x0.x, x0.y, x0.z, x0.w}, xb[4] = {x1.x, x1.y, x1.z, x1.w};
-  const float ya[4] = {y0.x, y0.y, y0.z, y0.w}, yb[4] = {y1.x, y1.y, y1.z, y1.w};
-  const float h2 = info.cell_m * info.cell_m;
+  const float xa[4] = {xm.x, xm.y, xm.z, xm.w}, xb[4] = {xp.x, xp.y, xp.z, xp.w};
+  const float ya[4] = {ym.x, ym.y, ym.z, ym.w}, yb[4] = {yp.x, yp.y, yp.z, yp.w};
+  const float zv[4] = {zc.x, zc.y, zc.z, zc.w};
+  const ClassStencil* table = t.e + 16 * class_of(i, d.n0) + 4 * class_of(j, d.n1);
+  const double inner = table[d.n2 >= 4 ? 1 : 2].inv, first = table[class_of(0, d.n2)].inv, last = table[3].inv;
+  const float vc = t.e[0].vc;
+  const int cells = (d.n2 + (odd ? 0 : 1)) / 2 - m0;          // how many of the four exist
+  const int last_n = (d.n2 & 1) == (odd ? 0 : 1) ? cells - 1 : -1;  // the one at k = n2 - 1, if it has this parity
   float out[4];
 #pragma unroll
   for (int n = 0; n < 4; ++n) {
-    const int k = 2 * (m0 + n) + P;
-    out[n] = qv[n];
-    if (k >= nz) continue;
-    const float sq = ((((xa[n] + xb[n]) + ya[n]) + yb[n]) + zs[n + P]) + zs[n + 1 + P];
-    const float x = sq - h2 * rv[n];  // (cell_m * cell_m) * rhs, as relaxed_uniform forms the source
-    float target = div6_core(x);
-    if (k == 0 || k == nz - 1 || !div6_in_range(x)) {
-      const float c0 = k > 0 ? 1.0f : (info.open_lo[2] == 1 ? ghost_coupling(info) : 0.0f);
-      const float c1 = k < nz - 1 ? 1.0f : (info.open_hi[2] == 1 ? ghost_coupling(info) : 0.0f);
-      target = x / ((4.0f + c0) + c1);  // neighbor_sum_uniform's couplings: 4 over x and y, then the z faces
-    }
-    out[n] = qv[n] + relaxation * (target - qv[n]);
+    const float zm = odd ? zv[n] : (n == 0 ? far : zv[n > 0 ? n - 1 : 0]);
+    const float zp = odd ? (n == 3 ? far : zv[n < 3 ? n + 1 : 3]) : zv[n];
+    const float sq = plain_sum(x0 ? xa[n] : 0.0f, x1 ? xb[n] : 0.0f, y0 ? ya[n] : 0.0f, y1 ? yb[n] : 0.0f, zm, zp);
+    const double inv = n == last_n ? last : (n == 0 && m0 == 0 && !odd ? first : inner);
+    const float value = qv[n] + relaxation * (quotient(sq - vc * rv[n], inv) - qv[n]);
+    out[n] = n < cells ? value : qv[n];
   }
   *reinterpret_cast<float4*>(qs + own) = make_float4(out[0], out[1], out[2], out[3]);
 }
 
-__global__ void k_rb_split4(PlumeGridInfo info, int H, float* __restrict__ qs, const float* __restrict__ rs, int color,
-                            float relaxation) {
+// k_residual_restrict with the fine level in split storage, four coarse cells kc0 .. kc0 + 3 per thread. The children of
+// coarse cell kc sit at half index m = kc in both colours' rows (fk = 2 kc and 2 kc + 1 are one of each colour). The
+// thread loads both colours' 16-byte rows of its two by two child rows once: they are each other's x, y and z
+// neighbours; around them it loads the rows beyond in x and y and the value beyond the four that an end's z neighbour
+// needs. Each coarse cell adds its children in the reference's order (di, dj, dk). Uniform levels. Bound by load latency,
+// so by the warps in flight: measured on B200 at 256x384x256, the 4-cycle solve takes 2.223 ms at four blocks of 64
+// registers per SM (a few spilled), 2.294 ms at three of 80, 2.298 ms at two; with two coarse cells per thread 2.269 ms
+// at best.
+__global__ void __launch_bounds__(256, 4)
+    k_residual_restrict_split(const __grid_constant__ LevelTable t, Dims fd, int H, const float* __restrict__ qs,
+                              const float* __restrict__ rs, Dims coarse, float* __restrict__ coarse_rhs,
+                              float* __restrict__ coarse_q) {
   wait_for_previous_grid();
-  const int nx = info.dims[0], ny = info.dims[1], nz = info.dims[2];
   const int i = blockIdx.z, j = blockIdx.y * blockDim.y + threadIdx.y;
   const int m0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
-  if (j >= ny || m0 >= H) return;
-  const int p = (i + j + color) & 1;  // cell k = 2 m + p
-  const long plane = (long)ny * H;
-  const long own = ((long)(color * nx + i) * ny + j) * H + m0;
-  const long oth = ((long)((1 - color) * nx + i) * ny + j) * H + m0;
-  // the other colour is not written by this pass
-  if (i > 0 && i < nx - 1 && j > 0 && j < ny - 1) {  // the same for a whole row: one branch per warp
-    if (p == 0) split_row_interior<0>(info, H, qs, rs, own, oth, plane, m0, relaxation);
-    else split_row_interior<1>(info, H, qs, rs, own, oth, plane, m0, relaxation);
-    return;
-  }
-  const float4 q4 = ld4(qs + own), r4 = ldg4(rs + own);
-  const float4 x0 = ldg4(qs + (i > 0 ? oth - plane : oth)), x1 = ldg4(qs + (i < nx - 1 ? oth + plane : oth));
-  const float4 y0 = ldg4(qs + (j > 0 ? oth - H : oth)), y1 = ldg4(qs + (j < ny - 1 ? oth + H : oth));
-  const float4 zc = ldg4(qs + oth);
-  const int mz = p == 0 ? m0 - 1 : m0 + 4;
-  const float zx = mz >= 0 && mz < H ? __ldg(qs + oth - m0 + mz) : 0.0f;
-  const float qv[4] = {q4.x, q4.y, q4.z, q4.w}, rv[4] = {r4.x, r4.y, r4.z, r4.w};
-  const float xa[4] = {x0.x, x0.y, x0.z, x0.w}, xb[4] = {x1.x, x1.y, x1.z, x1.w};
-  const float ya[4] = {y0.x, y0.y, y0.z, y0.w}, yb[4] = {y1.x, y1.y, y1.z, y1.w};
-  const float zs[6] = {zx, zc.x, zc.y, zc.z, zc.w, zx};  // the other colour's row at m0 - 1 .. m0 + 4
-  const float ghost = ghost_coupling(info);
-  float out[4] = {qv[0], qv[1], qv[2], qv[3]};
+  if (j >= coarse.n1 || m0 >= coarse.n2) return;
+  const long plane = (long)fd.n1 * H, colour = (long)fd.n0 * plane;
+  const bool two_i = 2 * i + 1 < fd.n0, two_j = 2 * j + 1 < fd.n1;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const long corner = (2L * i * fd.n1 + 2 * j) * H + m0;
+  // own[di][dj][p]: the child row's cells of parity p along z; (2 i + di + 2 j + dj) & 1 == (di + dj) & 1, so they have
+  // the colour (di + dj + p) & 1
+  long row[2][2];
+  Quad own[2][2][2];
 #pragma unroll
-  for (int n = 0; n < 4; ++n) {
-    const int k = 2 * (m0 + n) + p;
-    if (k >= nz) continue;
-    const float zm = p ? zs[n + 1] : zs[n], zp = p ? zs[n + 2] : zs[n + 1];  // at m - 1 + p and m + p
-    auto load = [&](int a, int b, int c) {
-      return a < i ? xa[n] : (a > i ? xb[n] : (b < j ? ya[n] : (b > j ? yb[n] : (c < k ? zm : zp))));
-    };
-    float value;
-    if (relax_cell(true, info, ghost, i, j, k, qv[n], rv[n], relaxation, load, value)) out[n] = value;
-  }
-  *reinterpret_cast<float4*>(qs + own) = make_float4(out[0], out[1], out[2], out[3]);
-}
-
-// The natural-layout colour pass (k_rb_colour) with four consecutive cells of a row per thread, two of them of
-// the colour: 16-byte loads of the row, of its four neighbouring rows and of rhs, and the one value beyond the
-// four that the row's parity needs. The other colour's two values are stored back unchanged: this pass never
-// writes them, so any thread reading them sees the same floats. Every update is relax_cell's. Rows of a
-// multiple of four cells, 16-byte-aligned arrays.
-// k_rb_colour4's two cells of a row with all four x and y neighbours on a uniform level, with split_row_interior's
-// straight-line arithmetic (the value beyond the row's ends reads 0).
-template <int P>
-__device__ __forceinline__ void colour4_row_interior(const PlumeGridInfo& info, float* __restrict__ q,
-                                                     const float* __restrict__ rhs, long row, long plane, int k0,
-                                                     float relaxation) {
-  const int nz = info.dims[2];
-  const float4 c4 = ld4(q + row), r4 = ldg4(rhs + row);
-  const float4 x0 = ld4(q + row - plane), x1 = ld4(q + row + plane);
-  const float4 y0 = ld4(q + row - nz), y1 = ld4(q + row + nz);
-  const int ze = P == 0 ? k0 - 1 : k0 + 4;
-  const float zx = (P == 0 ? ze >= 0 : ze < nz) ? q[row - k0 + ze] : 0.0f;
-  const float cv[4] = {c4.x, c4.y, c4.z, c4.w}, rv[4] = {r4.x, r4.y, r4.z, r4.w};
-  const float xa[4] = {x0.x, x0.y, x0.z, x0.w}, xb[4] = {x1.x, x1.y, x1.z, x1.w};
-  const float ya[4] = {y0.x, y0.y, y0.z, y0.w}, yb[4] = {y1.x, y1.y, y1.z, y1.w};
-  const float h2 = info.cell_m * info.cell_m;
-  float out[4] = {cv[0], cv[1], cv[2], cv[3]};
+  for (int di = 0; di < 2; ++di)
 #pragma unroll
-  for (int n = 0; n < 2; ++n) {
-    const int a = P + 2 * n, k = k0 + a;
-    const float zm = a == 0 ? zx : cv[a > 0 ? a - 1 : 0], zp = a == 3 ? zx : cv[a < 3 ? a + 1 : 3];
-    const float sq = ((((xa[a] + xb[a]) + ya[a]) + yb[a]) + zm) + zp;
-    const float x = sq - h2 * rv[a];
-    float target = div6_core(x);
-    if (k == 0 || k == nz - 1 || !div6_in_range(x)) {
-      const float c0 = k > 0 ? 1.0f : (info.open_lo[2] == 1 ? ghost_coupling(info) : 0.0f);
-      const float c1 = k < nz - 1 ? 1.0f : (info.open_hi[2] == 1 ? ghost_coupling(info) : 0.0f);
-      target = x / ((4.0f + c0) + c1);
+    for (int dj = 0; dj < 2; ++dj) {  // a missing child row: the first one's, its value never used
+      row[di][dj] = corner + (di && two_i ? plane : 0) + (dj && two_j ? H : 0);
+#pragma unroll
+      for (int p = 0; p < 2; ++p) own[di][dj][p] = Quad(ldg4(qs + ((di + dj + p) & 1) * colour + row[di][dj]));
     }
-    out[a] = cv[a] + relaxation * (target - cv[a]);
-  }
-  *reinterpret_cast<float4*>(q + row) = make_float4(out[0], out[1], out[2], out[3]);
-}
-
-template <bool UNIFORM>
-__global__ void k_rb_colour4(PlumeGridInfo info, float* __restrict__ q, const float* __restrict__ rhs, int color,
-                             float relaxation) {
-  wait_for_previous_grid();
-  const int nx = info.dims[0], ny = info.dims[1], nz = info.dims[2];
-  const int i = blockIdx.z, j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
-  if (j >= ny || k0 >= nz) return;
-  const int p = (i + j + color) & 1;  // this colour's cells: k0 + p and k0 + p + 2
-  const long plane = (long)ny * nz, row = ((long)i * ny + j) * nz + k0;
-  if (UNIFORM && i > 0 && i < nx - 1 && j > 0 && j < ny - 1) {  // the same for a whole row
-    if (p == 0) colour4_row_interior<0>(info, q, rhs, row, plane, k0, relaxation);
-    else colour4_row_interior<1>(info, q, rhs, row, plane, k0, relaxation);
-    return;
-  }
-  const float4 c4 = ld4(q + row), r4 = ldg4(rhs + row);
-  const float4 x0 = ld4(q + (i > 0 ? row - plane : row)), x1 = ld4(q + (i < nx - 1 ? row + plane : row));
-  const float4 y0 = ld4(q + (j > 0 ? row - nz : row)), y1 = ld4(q + (j < ny - 1 ? row + nz : row));
-  const int ze = p == 0 ? k0 - 1 : k0 + 4;
-  const float zx = ze >= 0 && ze < nz ? q[row - k0 + ze] : 0.0f;
-  const float cv[4] = {c4.x, c4.y, c4.z, c4.w}, rv[4] = {r4.x, r4.y, r4.z, r4.w};
-  const float xa[4] = {x0.x, x0.y, x0.z, x0.w}, xb[4] = {x1.x, x1.y, x1.z, x1.w};
-  const float ya[4] = {y0.x, y0.y, y0.z, y0.w}, yb[4] = {y1.x, y1.y, y1.z, y1.w};
-  const float ghost = ghost_coupling(info);
-  float out[4] = {cv[0], cv[1], cv[2], cv[3]};
-#pragma unroll
-  for (int n = 0; n < 2; ++n) {
-#pragma unroll
-    for (int pp = 0; pp < 2; ++pp) {  // a = p + 2 n with p known per thread: both cases unrolled
-      if (pp != p) continue;
-      const int a = pp + 2 * n, k = k0 + a;
-      const float zm = a == 0 ? zx : cv[a > 0 ? a - 1 : 0], zp = a == 3 ? zx : cv[a < 3 ? a + 1 : 3];
-      auto load = [&](int aa, int b, int c) {
-        return aa < i ? xa[a] : (aa > i ? xb[a] : (b < j ? ya[a] : (b > j ? yb[a] : (c < k ? zm : zp))));
-      };
-      float value;
-      if (relax_cell(UNIFORM, info, ghost, i, j, k, cv[a], rv[a], relaxation, load, value)) out[a] = value;
-    }
-  }
-  *reinterpret_cast<float4*>(q + row) = make_float4(out[0], out[1], out[2], out[3]);
-}
-
-// k_residual_restrict with the fine level in split storage, V (2 or 4) coarse cells kc0 .. kc0 + V - 1 per
-// thread. The children of coarse cell kc sit at half index m = kc in both colours' rows (fk = 2 kc and
-// 2 kc + 1 are one of each colour), so for each child (di, dj, dk) of the V cells the thread loads, as 8- or
-// 16-byte rows at m = kc0 .., the child's own row and rhs, the other colour's row (its z neighbours) and the
-// other colour's four neighbouring rows, plus the value beyond the V that an end's z neighbour needs. Every
-// child's residual is residual_cell's on those values, and each coarse cell adds its children in the
-// reference's order (di, dj, dk).
-template <int V>
-struct Row {
-  float v[V];
-};
-template <int V>
-__device__ __forceinline__ Row<V> ldg_row(const float* p) {
-  Row<V> r;
-  if constexpr (V == 4) {
-    const float4 a = ldg4(p);
-    r.v[0] = a.x, r.v[1] = a.y, r.v[2] = a.z, r.v[3] = a.w;
-  } else {
-    const float2 a = __ldg(reinterpret_cast<const float2*>(p));
-    r.v[0] = a.x, r.v[1] = a.y;
-  }
-  return r;
-}
-
-#ifndef PLUME_RESTRICT_MINB
-#define PLUME_RESTRICT_MINB 3
-#endif
-#ifndef PLUME_RESTRICT_CELLS
-#define PLUME_RESTRICT_CELLS 4
-#endif
-template <int V, bool UNIFORM>
-__global__ void __launch_bounds__(256, PLUME_RESTRICT_MINB)
-    k_residual_restrict_split(PlumeGridInfo fine, int H, const float* __restrict__ qs, const float* __restrict__ rs,
-                              Dims coarse, float* __restrict__ coarse_rhs, float* __restrict__ coarse_q) {
-  wait_for_previous_grid();
-  const int i = blockIdx.z, j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int kc0 = V * (blockIdx.x * blockDim.x + threadIdx.x);
-  if (j >= coarse.n1 || kc0 >= coarse.n2) return;
-  const Dims fd = dims_of(fine);
-  constexpr bool uniform = UNIFORM;  // the level's couplings are all 1 (is_uniform), chosen on the host
-  const float ghost = ghost_coupling(fine);
-  const long colour_floats = (long)fd.n0 * fd.n1 * H;
-  auto row = [&](int c, int a, int b) {  // (a, b)'s row of colour c at m = kc0, a and b clamped into the level
-    a = imin_(imax_(a, 0), fd.n0 - 1);
-    b = imin_(imax_(b, 0), fd.n1 - 1);
-    return c * colour_floats + ((long)a * fd.n1 + b) * H + kc0;
-  };
-  float total[V], count[V];
-#pragma unroll
-  for (int n = 0; n < V; ++n) total[n] = count[n] = 0.0f;
+  float total[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  const double inv_vc = t.e[0].inv_vc;
+  const int front = class_of(0, fd.n2), inner = fd.n2 >= 4 ? 1 : 2, last_m = (fd.n2 - 1) >> 1, last_p = (fd.n2 - 1) & 1;
 #pragma unroll
   for (int di = 0; di < 2; ++di)
 #pragma unroll
     for (int dj = 0; dj < 2; ++dj) {
       const int fi = 2 * i + di, fj = 2 * j + dj;
-      if (fi >= fd.n0 || fj >= fd.n1) continue;
-      const bool xy_interior = uniform && fi > 0 && fi < fd.n0 - 1 && fj > 0 && fj < fd.n1 - 1;
-      const int c0 = (fi + fj) & 1;  // the colour of child dk = 0; child dk = 1 has the other
+      const bool there = (di == 0 || two_i) && (dj == 0 || two_j);
+      const bool x0 = fi > 0, x1 = fi < fd.n0 - 1, y0 = fj > 0, y1 = fj < fd.n1 - 1;
+      const ClassStencil* table = t.e + 16 * class_of(imin_(fi, fd.n0 - 1), fd.n0) + 4 * class_of(imin_(fj, fd.n1 - 1), fd.n1);
+      const float sc_inner = table[inner].sc, sc_front = table[front].sc, sc_last = table[3].sc;
 #pragma unroll
-      for (int dk = 0; dk < 2; ++dk) {
-        const int cc = dk == 0 ? c0 : 1 - c0, oc = 1 - cc;
-        const Row<V> own = ldg_row<V>(qs + row(cc, fi, fj)), rhs = ldg_row<V>(rs + row(cc, fi, fj));
-        const Row<V> other = ldg_row<V>(qs + row(oc, fi, fj));
-        const Row<V> xm = ldg_row<V>(qs + row(oc, fi - 1, fj)), xp = ldg_row<V>(qs + row(oc, fi + 1, fj));
-        const Row<V> ym = ldg_row<V>(qs + row(oc, fi, fj - 1)), yp = ldg_row<V>(qs + row(oc, fi, fj + 1));
-        // z neighbours in the other colour's row: child dk = 0 (fk = 2 kc) at m = kc - 1 and kc, child dk = 1
-        // (fk = 2 kc + 1) at m = kc and kc + 1; the first needs m = kc0 - 1, the second m = kc0 + V
-        const float beyond = dk == 0 ? (kc0 >= 1 ? __ldg(qs + row(oc, fi, fj) - 1) : 0.0f)
-                                     : (kc0 + V < H ? __ldg(qs + row(oc, fi, fj) + V) : 0.0f);
+      for (int p = 0; p < 2; ++p) {
+        const long mine = ((di + dj + p) & 1) * colour + row[di][dj], c = ((di + dj + p + 1) & 1) * colour + row[di][dj];
+        Quad xm, xp, ym, yp;
+        if (di == 0) {
+          const float4 v = ldg4(qs + (x0 ? c - plane : c));
+          xm = Quad(x0 ? v : zero);
+          xp = x1 ? own[1][dj][p] : Quad(zero);  // the same cells one plane on have the other colour
+        } else {
+          const float4 v = ldg4(qs + (x1 ? c + plane : c));
+          xm = own[0][dj][p];
+          xp = Quad(x1 ? v : zero);
+        }
+        if (dj == 0) {
+          const float4 v = ldg4(qs + (y0 ? c - H : c));
+          ym = Quad(y0 ? v : zero);
+          yp = y1 ? own[di][1][p] : Quad(zero);
+        } else {
+          const float4 v = ldg4(qs + (y1 ? c + H : c));
+          ym = own[di][0][p];
+          yp = Quad(y1 ? v : zero);
+        }
+        // z neighbours at m - 1 and m (p = 0) or m and m + 1 (p = 1) of the other parity's row; padding slots hold 0
+        const bool has_far = p == 0 ? m0 > 0 : m0 + 4 < H;
+        const float far_value = __ldg(qs + c + (has_far ? (p == 0 ? -1 : 4) : 0)), far = has_far ? far_value : 0.0f;
+        const Quad r(ldg4(rs + mine));
+        const float* o = own[di][dj][1 - p].v;
 #pragma unroll
-        for (int n = 0; n < V; ++n) {
-          const int fk = 2 * (kc0 + n) + dk;
-          if (fk >= fd.n2) continue;
-          const float zm = dk == 0 ? (n == 0 ? beyond : other.v[n > 0 ? n - 1 : 0]) : other.v[n];
-          const float zp = dk == 0 ? other.v[n] : (n == V - 1 ? beyond : other.v[n < V - 1 ? n + 1 : V - 1]);
-          if (xy_interior) {
-            total[n] = total[n] + residual_xy_interior(fine, ghost, fk, own.v[n], rhs.v[n], xm.v[n], xp.v[n], ym.v[n],
-                                                       yp.v[n], zm, zp);
-            count[n] = count[n] + 1.0f;
-            continue;
-          }
-          auto load = [&](int a, int b, int c) {
-            return a < fi ? xm.v[n]
-                          : (a > fi ? xp.v[n] : (b < fj ? ym.v[n] : (b > fj ? yp.v[n] : (c < fk ? zm : zp))));
-          };
-          total[n] = total[n] + residual_cell(uniform, fine, ghost, fi, fj, fk, own.v[n], rhs.v[n], load);
-          count[n] = count[n] + 1.0f;
+        for (int n = 0; n < 4; ++n) {
+          const float zm = p == 0 ? (n == 0 ? far : o[n > 0 ? n - 1 : 0]) : o[n];
+          const float zp = p == 0 ? o[n] : (n == 3 ? far : o[n < 3 ? n + 1 : 3]);
+          const float sc = p == last_p && m0 + n == last_m ? sc_last : (p == 0 && n == 0 && m0 == 0 ? sc_front : sc_inner);
+          const float sq = plain_sum(xm.v[n], xp.v[n], ym.v[n], yp.v[n], zm, zp);
+          const float sum = total[n] + (r.v[n] - quotient(sq - sc * own[di][dj][p].v[n], inv_vc));
+          total[n] = there && 2 * (m0 + n) + p < fd.n2 ? sum : total[n];
         }
       }
     }
+  const float share = (two_i ? 0.5f : 1.0f) * (two_j ? 0.5f : 1.0f);
 #pragma unroll
-  for (int n = 0; n < V; ++n) {
-    if (kc0 + n >= coarse.n2) break;
-    const int out = at(coarse, i, j, kc0 + n);
-    coarse_rhs[out] = divide(total[n], divisor(count[n]));  // count is 1, 2, 4 or 8
+  for (int n = 0; n < 4; ++n) {
+    if (m0 + n >= coarse.n2) break;
+    const int out = at(coarse, i, j, m0 + n);
+    coarse_rhs[out] = total[n] * (2 * (m0 + n) + 1 < fd.n2 ? 0.5f * share : share);  // / 1, 2, 4 or 8: the same float
     coarse_q[out] = 0.0f;
   }
 }
 
-// k_prolong_add with the fine level in split storage, four cells of a row per thread: thread (c, i, j, m0)
+// k_prolong_rows4 with the fine level in split storage, four cells of a row per thread: thread (c, i, j, m0)
 // adds to its cells m0 .. m0 + 3 of colour c. The four share the coarse sample's x and y axes; along z they
 // read six consecutive coarse columns (m0 - 1 + p .. m0 + 4 + p, clamped), each blended in x then y once
 // (sample_index_space's first lerps, which run per column in that order), and each cell blends its two
@@ -1107,54 +1113,42 @@ static void launch_tiled(const PlumeGridInfo& info, Pressure& q, const float* rh
     k_rb_sweep<PROLONG, false><<<tile_grid(info), SWEEP_THREADS, 0, st>>>(info, q.cur, q.other, rhs, relaxation, coarse_q, cd);
 }
 
-// Levels of at least this many cells (q and rhs over 64 MB) sweep two planes per thread (k_rb_colour_pair).
-// PLUME_PAIR_MIN_CELLS overrides the threshold (for measurements).
-static const long RB_PAIR_MIN_CELLS = [] {
-  const char* v = getenv("PLUME_PAIR_MIN_CELLS");
-  return v ? atol(v) : 1L << 23;
-}();
-// Smaller levels with rows of a multiple of four cells sweep four cells of a row per thread (k_rb_colour4);
-// PLUME_COLOUR4=0 keeps one cell per thread.
-static const bool g_colour4 = [] {
-  const char* v = getenv("PLUME_COLOUR4");
-  return !(v && v[0] == '0');
-}();
+static bool rows4(const Dims& d, const void* a, const void* b) {
+  return d.n2 % 4 == 0 && (((uintptr_t)a | (uintptr_t)b) & 15) == 0;
+}
 
-static int colour_sweep(const PlumeGridInfo& info, float* q, const float* rhs, float relaxation, cudaStream_t st) {
+static int colour_sweep(const PlumeGridInfo& info, const LevelTable& table, float* q, const float* rhs, float relaxation,
+                        cudaStream_t st) {
   const Dims d = dims_of(info);
-  if (cells_of(info) >= RB_PAIR_MIN_CELLS) {
-    const dim3 grid(((d.n2 + 1) / 2 + TZ - 1) / TZ, (d.n1 + TY - 1) / TY, (d.n0 + 1) / 2);
-    for (int color = 0; color < 2; ++color) {
-      int status = uniform_level(info) ? launch_solve_kernel(k_rb_colour_pair<true>, grid, cell_block(), 0, st,
-                                                             "red-black colour", info, q, rhs, color, relaxation)
-                                       : launch_solve_kernel(k_rb_colour_pair<false>, grid, cell_block(), 0, st,
-                                                             "red-black colour", info, q, rhs, color, relaxation);
-      if (status != PLUME_OK) return status;
-    }
-    return PLUME_OK;
-  }
-  if (g_colour4 && d.n2 % 4 == 0 && (((uintptr_t)q | (uintptr_t)rhs) & 15) == 0) {
-    const dim3 grid((d.n2 / 4 + TZ - 1) / TZ, (d.n1 + TY - 1) / TY, d.n0);
-    for (int color = 0; color < 2; ++color) {
-      int status = uniform_level(info) ? launch_solve_kernel(k_rb_colour4<true>, grid, cell_block(), 0, st,
-                                                             "red-black colour", info, q, rhs, color, relaxation)
-                                       : launch_solve_kernel(k_rb_colour4<false>, grid, cell_block(), 0, st,
-                                                             "red-black colour", info, q, rhs, color, relaxation);
-      if (status != PLUME_OK) return status;
-    }
-    return PLUME_OK;
-  }
-  const dim3 grid(((d.n2 + 1) / 2 + TZ - 1) / TZ, (d.n1 + TY - 1) / TY, d.n0);
+  const bool uniform = uniform_level(info) && cells_of(info) > 1, wide = rows4(d, q, rhs);
+  const dim3 grid(((wide ? d.n2 / 4 : (d.n2 + 1) / 2) + TZ - 1) / TZ, (d.n1 + TY - 1) / TY, d.n0);
+  auto kernel = wide ? (uniform ? k_colour_rows4<true> : k_colour_rows4<false>)
+                     : (uniform ? k_colour_cells<true> : k_colour_cells<false>);
   for (int color = 0; color < 2; ++color) {
-    const float* none = nullptr;
-    int status = uniform_level(info)
-                     ? launch_solve_kernel(k_rb_colour<true>, grid, cell_block(), 0, st, "red-black colour", info, q, rhs,
-                                           color, relaxation, none, Dims{1, 1, 1})
-                     : launch_solve_kernel(k_rb_colour<false>, grid, cell_block(), 0, st, "red-black colour", info, q,
-                                           rhs, color, relaxation, none, Dims{1, 1, 1});
+    int status = launch_solve_kernel(kernel, grid, cell_block(), 0, st, "red-black colour", table, d, q, rhs, color, relaxation);
     if (status != PLUME_OK) return status;
   }
   return PLUME_OK;
+}
+
+static int launch_restrict(const PlumeGridInfo& info, const LevelTable& table, const float* q, const float* rhs,
+                           const PlumeLevel& coarse, cudaStream_t st) {
+  const Dims d = dims_of(info), cd = dims_of(coarse.info);
+  const bool uniform = uniform_level(info);
+  const bool wide = rows4(d, q, rhs) && (((uintptr_t)coarse.rhs | (uintptr_t)coarse.q) & 7) == 0;
+  const dim3 grid(((d.n2 + 3) / 4 + TZ - 1) / TZ, (cd.n1 + TY - 1) / TY, cd.n0);
+  auto kernel = wide ? (uniform ? k_residual_restrict<true, true> : k_residual_restrict<false, true>)
+                     : (uniform ? k_residual_restrict<true, false> : k_residual_restrict<false, false>);
+  return launch_solve_kernel(kernel, grid, cell_block(), 0, st, "residual and restriction", table, d, q, rhs, cd, coarse.rhs,
+                             coarse.q);
+}
+
+static int launch_prolong(const PlumeGridInfo& info, float* q, const float* coarse_q, const PlumeGridInfo& coarse,
+                          cudaStream_t st) {
+  const Dims d = dims_of(info), cd = dims_of(coarse);
+  const bool wide = rows4(d, q, q) && ((uintptr_t)coarse_q & 7) == 0;
+  const dim3 grid(((d.n2 + 3) / 4 + TZ - 1) / TZ, (d.n1 + TY - 1) / TY, d.n0);
+  return launch_solve_kernel(wide ? k_prolong_rows4<true> : k_prolong_rows4<false>, grid, cell_block(), 0, st, "prolong", cd, d, coarse_q, q);
 }
 
 // The split top level's prolongation takes both colours of a row's four half indices per thread when the
@@ -1192,10 +1186,11 @@ static int split_sweeps(const PlumeGridInfo& info, const SplitTop& sp, int sweep
     if (status != PLUME_OK) return status;
   }
   const dim3 grid((sp.H / 4 + TZ - 1) / TZ, (d.n1 + TY - 1) / TY, d.n0);
+  const LevelTable table = level_table(info);
   for (int s = 0; s < sweeps; ++s)
     for (int color = 0; color < 2; ++color) {
-      int status = launch_solve_kernel(k_rb_split4, grid, cell_block(), 0, st, "red-black colour (split)", info,
-                                       sp.H, sp.q, (const float*)sp.rhs, color, 1.0f);
+      int status = launch_solve_kernel(k_rb_split4, grid, cell_block(), 0, st, "red-black colour (split)", table, d, sp.H,
+                                       sp.q, (const float*)sp.rhs, color, 1.0f);
       if (status != PLUME_OK) return status;
     }
   return PLUME_OK;
@@ -1207,12 +1202,11 @@ static int sweeps_with_prolong(const PlumeGridInfo& info, Pressure& q, const flo
                                const float* coarse_q, const PlumeGridInfo* coarse, cudaStream_t st) {
   int s = 0;
   const bool tiled = cells_of(info) >= g_tiled_min_cells;
+  const LevelTable table = level_table(info);
   if (coarse) {
     const Dims cd = dims_of(*coarse);
     if (sweeps == 0 || !tiled) {
-      const Dims fd = dims_of(info);
-      int status = launch_solve_kernel(k_prolong_add, cell_grid(fd.n0, fd.n1, fd.n2), cell_block(), 0, st, "prolong",
-                                       cd, fd, coarse_q, q.cur);
+      int status = launch_prolong(info, q.cur, coarse_q, *coarse, st);
       if (status != PLUME_OK) return status;
     } else {
       launch_tiled<true>(info, q, rhs, relaxation, coarse_q, cd, st);
@@ -1229,7 +1223,7 @@ static int sweeps_with_prolong(const PlumeGridInfo& info, Pressure& q, const flo
       if (status != PLUME_OK) return status;
       q.flip();
     } else {
-      int status = colour_sweep(info, q.cur, rhs, relaxation, st);
+      int status = colour_sweep(info, table, q.cur, rhs, relaxation, st);
       if (status != PLUME_OK) return status;
     }
   }
@@ -1378,15 +1372,10 @@ static int v_cycle(const PlumeLevel* levels, int count, int index, Pressure& q, 
     if (status != PLUME_OK) return status;
     const PlumeLevel& coarse = levels[1];
     const Dims cd = dims_of(coarse.info);
-    constexpr int V = PLUME_RESTRICT_CELLS;
-    const dim3 grid(((cd.n2 + V - 1) / V + TZ - 1) / TZ, (cd.n1 + TY - 1) / TY, cd.n0);
-    status = uniform_level(lv.info)
-                 ? launch_solve_kernel(k_residual_restrict_split<V, true>, grid, cell_block(), 0, st,
-                                       "residual and restriction (split)", lv.info, split->H, (const float*)split->q,
-                                       (const float*)split->rhs, cd, coarse.rhs, coarse.q)
-                 : launch_solve_kernel(k_residual_restrict_split<V, false>, grid, cell_block(), 0, st,
-                                       "residual and restriction (split)", lv.info, split->H, (const float*)split->q,
-                                       (const float*)split->rhs, cd, coarse.rhs, coarse.q);
+    const dim3 grid(((cd.n2 + 3) / 4 + TZ - 1) / TZ, (cd.n1 + TY - 1) / TY, cd.n0);
+    status = launch_solve_kernel(k_residual_restrict_split, grid, cell_block(), 0, st, "residual and restriction (split)",
+                                 level_table(lv.info), dims_of(lv.info), split->H, (const float*)split->q,
+                                 (const float*)split->rhs, cd, coarse.rhs, coarse.q);
     if (status != PLUME_OK) return status;
     Pressure coarse_q{coarse.q, coarse.residual};
     if ((status = v_cycle(levels, count, 1, coarse_q, plan, sweeps, st, coarse_f64)) != PLUME_OK) return status;
@@ -1417,10 +1406,7 @@ static int v_cycle(const PlumeLevel* levels, int count, int index, Pressure& q, 
   if (status != PLUME_OK) return status;
   const PlumeLevel& coarse = levels[index + 1];
   const Dims cd = dims_of(coarse.info);
-  if ((status = launch_solve_kernel(k_residual_restrict, cell_grid(cd.n0, cd.n1, cd.n2), cell_block(), 0, st,
-                                    "residual and restriction", lv.info, q.cur, lv.rhs, cd, coarse.rhs, coarse.q)) !=
-      PLUME_OK)
-    return status;
+  if ((status = launch_restrict(lv.info, level_table(lv.info), q.cur, lv.rhs, coarse, st)) != PLUME_OK) return status;
   Pressure coarse_q{coarse.q, coarse.residual};
   if ((status = v_cycle(levels, count, index + 1, coarse_q, plan, sweeps, st, coarse_f64)) != PLUME_OK)
     return status;

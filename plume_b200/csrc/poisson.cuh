@@ -158,19 +158,6 @@ __device__ __forceinline__ float residual_uniform(const PlumeGridInfo& info, flo
   return rhs - divide(sq - sc * q, divisor(info.cell_m * info.cell_m));
 }
 
-// residual_uniform for a cell whose four x and y neighbours all exist, at any k, from the neighbours passed in:
-// neighbor_sum_uniform's sums in its order (a missing z neighbour adds 0 and its face's coupling), so every value
-// is residual_uniform's.
-__device__ __forceinline__ float residual_xy_interior(const PlumeGridInfo& info, float ghost, int k, float q, float rhs,
-                                                      float x0, float x1, float y0, float y1, float zm, float zp) {
-  const bool lo = k > 0, hi = k < info.dims[2] - 1;
-  const float sq = (((((0.0f + x0) + x1) + y0) + y1) + (lo ? zm : 0.0f)) + (hi ? zp : 0.0f);
-  const float c0 = lo ? 1.0f : (info.open_lo[2] == 1 ? ghost : 0.0f);
-  const float c1 = hi ? 1.0f : (info.open_hi[2] == 1 ? ghost : 0.0f);
-  const float sc = (4.0f + c0) + c1;  // (((0 + 1) + 1) + 1) + 1 == 4 over x and y, then the two z faces
-  return rhs - divide(sq - sc * q, divisor(info.cell_m * info.cell_m));
-}
-
 // Either path, chosen per level.
 template <class Load>
 __device__ __forceinline__ bool relax_cell(bool uniform, const PlumeGridInfo& info, float ghost, int i, int j, int k,
