@@ -14,7 +14,7 @@
 #include <vector>
 
 #include "advect.cuh"
-#include "poisson.cuh"
+#include "stencil_table.cuh"
 
 namespace plume {
 
@@ -477,12 +477,76 @@ __device__ __forceinline__ float potential(int seed, int component, F3 p, float 
   return lerpf_(value_noise(seed, first, p), value_noise(seed, first + 3, p), blend);
 }
 
+// The turbulence potentials at the grid's edges, each formed once: component a sits at the middles of the edges along
+// axis a, and the push of a face is the differences of the four edges around it, so a potential serves up to four faces
+// (each face on its own would form four). The noise's lattice points lie scale_m / cell_m cells apart, so where that is
+// coarse their values come from a table of the six noise slices (three components, two times), each hashed once.
+struct EdgePotentials {
+  float* edge[3];      // (nx, ny+1, nz+1), (nx+1, ny, nz+1), (nx+1, ny+1, nz)
+  float* lattice;      // [component][slice][i][j][k], or null: hash the lattice points in place
+  Dims lattice_dims;
+  int seed;
+  float to_lattice, pattern_time;
+};
+
+__global__ void k_noise_lattice(EdgePotentials e) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int slab = blockIdx.z / e.lattice_dims.n0, i = blockIdx.z - slab * e.lattice_dims.n0;  // slab: component, slice
+  if (j >= e.lattice_dims.n1 || k >= e.lattice_dims.n2) return;
+  const int stream = TURBULENCE_STREAM + 3 * ((int)floorf(e.pattern_time) + slab % 2) + slab / 2;
+  const long points = (long)e.lattice_dims.n0 * e.lattice_dims.n1 * e.lattice_dims.n2;
+  e.lattice[slab * points + at(e.lattice_dims, i, j, k)] = lattice_value(e.seed, stream, i, j, k);
+}
+
+template <bool TABLE>
+__global__ void k_edge_potentials(PlumeGridInfo info, EdgePotentials e) {
+  const int nx = info.dims[0];
+  int i = blockIdx.z, axis = 0;  // slabs: nx of component 0, then nx + 1 of components 1 and 2
+  if (i >= nx) {
+    i -= nx;
+    axis = 1;
+    if (i >= nx + 1) {
+      i -= nx + 1;
+      axis = 2;
+    }
+  }
+  const Dims d{nx + (axis != 0), info.dims[1] + (axis != 1), info.dims[2] + (axis != 2)};
+  const int j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= d.n1 || k >= d.n2) return;
+  const F3 p = mul3(f3((float)i + (axis == 0 ? 0.5f : 0.0f), (float)j + (axis == 1 ? 0.5f : 0.0f),
+                       (float)k + (axis == 2 ? 0.5f : 0.0f)), e.to_lattice);
+  float value;
+  if constexpr (TABLE) {  // potential() with value_noise's floats, the lattice values read
+    const float fx = floorf(p[0]), fy = floorf(p[1]), fz = floorf(p[2]);
+    const float tx = fade(p[0] - fx), ty = fade(p[1] - fy), tz = fade(p[2] - fz);
+    const Dims& ld = e.lattice_dims;
+    const int sx = ld.n1 * ld.n2, sy = ld.n2;
+    const long points = (long)ld.n0 * sx;
+    const float* f = e.lattice + 2 * axis * points + at(ld, (int)fx, (int)fy, (int)fz);
+    float slice[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s, f += points) {
+      const float c00 = lerpf_(__ldg(f), __ldg(f + sx), tx), c10 = lerpf_(__ldg(f + sy), __ldg(f + sx + sy), tx);
+      const float c01 = lerpf_(__ldg(f + 1), __ldg(f + sx + 1), tx);
+      const float c11 = lerpf_(__ldg(f + sy + 1), __ldg(f + sx + sy + 1), tx);
+      slice[s] = lerpf_(lerpf_(c00, c10, ty), lerpf_(c01, c11, ty), tz);
+    }
+    value = lerpf_(slice[0], slice[1], fade(e.pattern_time - floorf(e.pattern_time)));
+  } else {
+    value = potential(e.seed, axis, p, e.pattern_time);
+  }
+  float* out = axis == 0 ? e.edge[0] : (axis == 1 ? e.edge[1] : e.edge[2]);
+  out[at(d, i, j, k)] = value;
+}
+
 struct FaceForces {
   int confinement;  // add the averaged push (add_face_push_kernel, vorticity.py:74-84)
   const float* push[3];
   int turbulence;   // turbulence_kernel (turbulence.py:35-53)
   int seed;
   float scale_m, strength, pattern_time;
+  const float* edge[3];  // k_edge_potentials' arrays, or null: the potentials formed in place
+  double inv_to_lattice; // 1 / (cell_m / scale_m), with the edge arrays
   int drag;         // drag_kernel (forces.py:34-37)
   float wind[3];
   float keep;
@@ -512,7 +576,16 @@ __device__ __forceinline__ float face_forces_value(const PlumeGridInfo& info, fl
     float average = 0.5f * (below + above);
     value = value + average * ff.dt;
   }
-  if (ff.turbulence) {
+  if (ff.turbulence && ff.edge[0]) {
+    constexpr int B = (AXIS + 1) % 3, C = (AXIS + 2) % 3;
+    const Dims db{info.dims[0] + (B != 0), info.dims[1] + (B != 1), info.dims[2] + (B != 2)};
+    const Dims dc{info.dims[0] + (C != 0), info.dims[1] + (C != 1), info.dims[2] + (C != 2)};
+    const int sb = B == 0 ? dc.n1 * dc.n2 : (B == 1 ? dc.n2 : 1), sc = C == 0 ? db.n1 * db.n2 : (C == 1 ? db.n2 : 1);
+    const float* on_c = ff.edge[C] + at(dc, i, j, k);
+    const float* on_b = ff.edge[B] + at(db, i, j, k);
+    const float curl = quotient((__ldg(on_c + sb) - __ldg(on_c)) - (__ldg(on_b + sc) - __ldg(on_b)), ff.inv_to_lattice);
+    value = value + ff.strength * curl * ff.dt;
+  } else if (ff.turbulence) {
     const F3 offset = AXIS == 0 ? f3(0.0f, 0.5f, 0.5f) : (AXIS == 1 ? f3(0.5f, 0.0f, 0.5f) : f3(0.5f, 0.5f, 0.0f));
     const F3 face = add3(f3((float)i, (float)j, (float)k), offset);
     constexpr int B = (AXIS + 1) % 3, C = (AXIS + 2) % 3;
@@ -583,6 +656,42 @@ __global__ void k_face_forces(PlumeGridInfo info, T* __restrict__ u, T* __restri
   if (axis == 0) face_forces_planes<0, PLANES>(info, u, i0, j, k, ff);
   else if (axis == 1) face_forces_planes<1, PLANES>(info, v, i0, j, k, ff);
   else face_forces_planes<2, PLANES>(info, w, i0, j, k, ff);
+}
+
+// Forms the turbulence potentials of `ff` at the edges in `scratch` (`floats` of them) and points `ff` at them, for grids
+// on which that pays: measured on B200, forces with turbulence FIGURES.
+static int launch_edge_potentials(const PlumeGridInfo& info, FaceForces& ff, float* scratch, long long floats,
+                                  cudaStream_t st) {
+  const int nx = info.dims[0], ny = info.dims[1], nz = info.dims[2];
+  const float to_lattice = info.cell_m / ff.scale_m;
+  const long long ex = (long long)nx * (ny + 1) * (nz + 1), ey = (long long)(nx + 1) * ny * (nz + 1);
+  const long long ez = (long long)(nx + 1) * (ny + 1) * nz;
+  if (!(to_lattice > 0.0f) || ex + ey + ez > floats || 3LL * nx + 2 > 65535) return PLUME_OK;  // the potentials are formed in place
+  EdgePotentials e{};
+  e.edge[0] = scratch;
+  e.edge[1] = scratch + ex;
+  e.edge[2] = scratch + ex + ey;
+  e.seed = ff.seed;
+  e.to_lattice = to_lattice;
+  e.pattern_time = ff.pattern_time;
+  // the lattice points around every edge: the largest coordinate's floor and the next one
+  const float far[3] = {(float)nx * to_lattice, (float)ny * to_lattice, (float)nz * to_lattice};
+  const bool small = far[0] < 4096.0f && far[1] < 4096.0f && far[2] < 4096.0f;
+  e.lattice_dims = small ? Dims{(int)far[0] + 2, (int)far[1] + 2, (int)far[2] + 2} : Dims{4098, 4098, 4098};
+  const long long points = 6LL * e.lattice_dims.n0 * e.lattice_dims.n1 * e.lattice_dims.n2;
+  const bool table = points <= (long long)nx * ny * nz / 2 && ex + ey + ez + points <= floats && 6 * e.lattice_dims.n0 <= 65535;
+  if (table) {
+    e.lattice = scratch + ex + ey + ez;
+    const dim3 grid((e.lattice_dims.n2 + TZ - 1) / TZ, (e.lattice_dims.n1 + TY - 1) / TY, 6 * e.lattice_dims.n0);
+    k_noise_lattice<<<grid, cell_block(), 0, st>>>(e);
+    CHECK_LAUNCH("noise lattice");
+  }
+  const dim3 grid((nz + 1 + TZ - 1) / TZ, (ny + 1 + TY - 1) / TY, 3 * nx + 2);
+  (table ? k_edge_potentials<true> : k_edge_potentials<false>)<<<grid, cell_block(), 0, st>>>(info, e);
+  CHECK_LAUNCH("edge potentials");
+  for (int a = 0; a < 3; ++a) ff.edge[a] = e.edge[a];
+  ff.inv_to_lattice = 1.0 / (double)to_lattice;
+  return PLUME_OK;
 }
 
 template <class T>
@@ -1629,6 +1738,10 @@ static int step(const PlumeStepState* s, const PlumeStepParams* p, void* stream)
     ff.scale_m = p->turbulence_scale_m;
     ff.strength = p->turbulence_strength;
     ff.pattern_time = p->turbulence_pattern_time;
+    // the advection's scratch is free until its passes run
+    if (s->advect_scratch &&
+        (status = launch_edge_potentials(info, ff, s->advect_scratch, plume_advect_scratch_floats(&info), st)) != PLUME_OK)
+      return status;
   }
   if (p->apply_drag) {
     ff.drag = 1;
