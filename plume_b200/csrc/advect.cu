@@ -101,9 +101,10 @@ __device__ __forceinline__ void ring_corners(const float* ring, int x, int inpla
 // Corners from global memory, indices clamped to the array as sample.py does.
 template <class T>
 __device__ __forceinline__ void global_corners(const T* __restrict__ f, const Dims& d, int x, int y, int z, float* a) {
-  const int x0 = imin_(x, d.n0 - 1), x1 = imin_(x + 1, d.n0 - 1);
-  const int y0 = imin_(y, d.n1 - 1), y1 = imin_(y + 1, d.n1 - 1);
-  const int z0 = imin_(z, d.n2 - 1), z1 = imin_(z + 1, d.n2 - 1);
+  // clamped before the step up: a coordinate beyond the int range has the largest int as its floor
+  const int x0 = imin_(x, d.n0 - 1), x1 = imin_(x0 + 1, d.n0 - 1);
+  const int y0 = imin_(y, d.n1 - 1), y1 = imin_(y0 + 1, d.n1 - 1);
+  const int z0 = imin_(z, d.n2 - 1), z1 = imin_(z0 + 1, d.n2 - 1);
   a[0] = ldg_f(f + at(d, x0, y0, z0));
   a[1] = ldg_f(f + at(d, x1, y0, z0));
   a[2] = ldg_f(f + at(d, x0, y1, z0));
@@ -140,7 +141,11 @@ __device__ __forceinline__ Dims group_dims(const PlumeGridInfo& info, int g) {
   return Dims{info.dims[0] + (g == 0), info.dims[1] + (g == 1), info.dims[2] + (g == 2)};
 }
 
-__device__ __forceinline__ float maxabs3(F3 v) { return fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fabsf(v[2])); }
+// Whether a trace by this velocity stays inside the staged planes: every component, each compared by itself, so that one
+// that is no number does not (a maximum would pass over it, and its coordinate's index would leave the ring).
+__device__ __forceinline__ bool within_reach(F3 v, float dt) {
+  return fabsf(v[0]) * dt < REACH && fabsf(v[1]) * dt < REACH && fabsf(v[2]) * dt < REACH;
+}
 
 // ---- velocity at a point (sample.py:74-82), from the staged ring or from global memory --------------------
 // The three components' axes are split once: x of v and w, y of u and w, z of u and v are the same
@@ -285,12 +290,12 @@ __device__ __forceinline__ void hat_at(const Args<T>& A, const float* vring, con
   const F3 p = add3(f3((float)x, (float)y, (float)z), off);
   const int inplane = y * RZ + z - rowbase;
   const F3 vp = ring_node<G>(vring, x, inplane);
-  bool fast = maxabs3(vp) * fabsf(A.dt) < REACH;
+  bool fast = within_reach(vp, fabsf(A.dt));
   F3 src = p;
   if (fast) {
     const F3 mid = sub3(p, mul3(vp, 0.5f * A.dt));
     const F3 vm = ring_velocity<Stride<G>::value>(vring, rowbase, mid);
-    fast = maxabs3(vm) * fabsf(A.dt) < REACH;
+    fast = within_reach(vm, fabsf(A.dt));
     src = sub3(p, mul3(vm, A.dt));
   }
   if (!fast) {
@@ -336,8 +341,9 @@ __device__ __noinline__ void back_global(const Args<T>& A, const float* hring, i
   const Ax gx = split(g[0]), gy = split(g[1]), gz = split(g[2]);
   float a[F][8];
   for (int c = 0; c < 8; ++c) {
-    const int cx = imin_(gx.i + (c & 1), gd.n0 - 1), cy = imin_(gy.i + ((c >> 1) & 1), gd.n1 - 1);
-    const int cz = imin_(gz.i + (c >> 2), gd.n2 - 1);
+    const int cx = imin_(imin_(gx.i, gd.n0 - 1) + (c & 1), gd.n0 - 1);
+    const int cy = imin_(imin_(gy.i, gd.n1 - 1) + ((c >> 1) & 1), gd.n1 - 1);
+    const int cz = imin_(imin_(gz.i, gd.n2 - 1) + (c >> 2), gd.n2 - 1);
     const bool staged = cx >= plane_lo && cx <= plane_lo + 2 && cy >= j0 - 1 && cy <= j0 + TY && cz >= k0 - 1 &&
                         cz <= k0 + TZ;
     if (staged) {
@@ -528,12 +534,12 @@ __device__ __forceinline__ void march(const Args<T>& A, int seg, float* sm) {
       const F3 p = add3(f3((float)i, (float)tj, (float)tk), off);
       const int inplane = tj * RZ + tk - rowbase;
       const F3 vp = ring_node<G>(vring, i, inplane);
-      bool fast = maxabs3(vp) * fabsf(A.dt) < REACH;
+      bool fast = within_reach(vp, fabsf(A.dt));
       float back[F];
       if (fast) {
         const F3 mid = sub3(p, mul3(vp, 0.5f * -A.dt));
         const F3 vm = ring_velocity<VS>(vring, rowbase, mid);
-        fast = maxabs3(vm) * fabsf(A.dt) < REACH;
+        fast = within_reach(vm, fabsf(A.dt));
         if (fast) {
           const F3 bsrc = sub3(p, mul3(vm, -A.dt));
           if (G == 3 && A.uses_outside == 1 && is_outside_open_face(bsrc, A.info)) {
