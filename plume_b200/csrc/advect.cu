@@ -30,6 +30,7 @@
 // each line in order and the lines in double. Temperature's dissipation (dissipate.py:10-15) is applied as
 // it is stored.
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 
 #include "advect.cuh"
@@ -37,8 +38,7 @@
 namespace plume {
 namespace mac {
 
-// Tile height: 8 rows (256 threads, four blocks per SM). Measured on B200 at 256x384x256, velocity advection:
-// 2.25 ms at 8 rows, 2.31 ms at 16 (512 threads, two blocks per SM).
+// Tile height of the scalar march, and rows of threads of the velocity march: 8 (256 threads).
 #ifndef PLUME_MAC_TY
 #define PLUME_MAC_TY 8
 #endif
@@ -55,8 +55,19 @@ constexpr int VR = 8;                                     // velocity ring: plan
 constexpr int SR = 4;                                     // smoke/temperature ring: planes i..i+2, i+3 landing
 constexpr int HR = 4;                                     // hat ring: planes i-1..i+1 read, i+2 written next
 constexpr float REACH = 0.98f;                            // trace reach (cells) served from shared memory
+// Floats after the last hat plane: where a coordinate's rounding step is a sixteenth of a cell or more (axes of 2^19), a
+// trace just under REACH ends a whole cell away, and the upper corner, of weight 0, lies one row further.
+constexpr int SLACK = HZ + 1;
 constexpr int RPN = RY * RZ;                              // staged elements per plane
 constexpr int STAGE_PER_THREAD = (RPN + NT - 1) / NT;
+// The velocity march's tile: EPT elements per thread, in rows TY apart.
+template <int EPT>
+struct March {
+  static constexpr int tile = EPT * TY, rows = tile + 4, staged = rows * RZ, plane = pad32(staged);  // staged plane
+  static constexpr int hat_rows = tile + 2, hat_plane = pad32(hat_rows * HZ), halo = hat_rows * HZ - EPT * NT;
+  static constexpr int per_thread = (staged + NT - 1) / NT;
+  static constexpr size_t smem = sizeof(float) * (3 * VR * plane + HR * hat_plane + SLACK);
+};
 
 __device__ __forceinline__ float lerpm(float a, float b, float t) { return __fmaf_rn(t, b - a, a); }
 
@@ -225,9 +236,8 @@ struct Stride {
   static constexpr int value = G == 3 ? RPN : RP;
 };
 
-template <int G>
+template <int G, int S = Stride<G>::value>
 __device__ __forceinline__ F3 ring_node(const float* vring, int x, int inplane) {
-  constexpr int S = Stride<G>::value;
   auto ring = [&](const float* r) {
     return [=](int dx, int dy, int dz) { return r[((x + dx) & (VR - 1)) * S + inplane + dy * RZ + dz]; };
   };
@@ -323,7 +333,7 @@ __device__ __forceinline__ void hat_at(const Args<T>& A, const float* vring, con
 // ---- the backward sample of hat (the reference's `back`) ---------------------------------------------------
 // From the hat ring when the backward trace stays inside it, else each corner's hat from wherever it is: the
 // ring for corners inside the staged hat planes, hat_global for the rest.
-template <int G, class T>
+template <int G, int ROWS, int PLANE, class T>
 __device__ __noinline__ void back_global(const Args<T>& A, const float* hring, int hbase, int j0, int k0, int plane_lo,
                                          int x, int y, int z, float* back) {
   constexpr int F = Fields<G>::count;
@@ -344,10 +354,10 @@ __device__ __noinline__ void back_global(const Args<T>& A, const float* hring, i
     const int cx = imin_(imin_(gx.i, gd.n0 - 1) + (c & 1), gd.n0 - 1);
     const int cy = imin_(imin_(gy.i, gd.n1 - 1) + ((c >> 1) & 1), gd.n1 - 1);
     const int cz = imin_(imin_(gz.i, gd.n2 - 1) + (c >> 2), gd.n2 - 1);
-    const bool staged = cx >= plane_lo && cx <= plane_lo + 2 && cy >= j0 - 1 && cy <= j0 + TY && cz >= k0 - 1 &&
+    const bool staged = cx >= plane_lo && cx <= plane_lo + 2 && cy >= j0 - 1 && cy <= j0 + ROWS && cz >= k0 - 1 &&
                         cz <= k0 + TZ;
     if (staged) {
-      for (int f = 0; f < F; ++f) a[f][c] = hring[(f * HR + (cx & (HR - 1))) * HP + cy * HZ + cz - hbase];
+      for (int f = 0; f < F; ++f) a[f][c] = hring[(f * HR + (cx & (HR - 1))) * PLANE + cy * HZ + cz - hbase];
     } else {
       float h[F], lo[F], hi[F];
       hat_global<G>(A, cx, cy, cz, h, lo, hi);
@@ -559,7 +569,7 @@ __device__ __forceinline__ void march(const Args<T>& A, int seg, float* sm) {
           }
         }
       }
-      if (!fast) back_global<G>(A, hring, hbase, j0, k0, i - 1, i, tj, tk, back);
+      if (!fast) back_global<G, TY, HP>(A, hring, hbase, j0, k0, i - 1, i, tj, tk, back);
       const size_t out = (size_t)i * plane_stride + (size_t)tj * gd.n2 + tk;
 #pragma unroll
       for (int f = 0; f < F; ++f) {
@@ -590,10 +600,312 @@ __device__ __forceinline__ void march(const Args<T>& A, int seg, float* sm) {
   }
 }
 
-// MINB: resident blocks per SM the kernel is compiled for (4 at 256 threads: at most 64 registers a thread;
-// 3: 80; 2: 128).
-template <class T, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_mac_velocity(Args<T> A) {
+// ---- the velocity march -----------------------------------------------------------------------------------------
+// One component (G) of the velocity by itself. The forward and the backward trace of an element start from the same
+// velocity and step half a cell either way, so both midpoint velocities are formed together when the element's hat
+// is, each operation once for the pair (two-wide fused multiply-adds: lane 0 forward, lane 1 backward, each lane the
+// scalar operation), and the backward trace's end point is kept until the correction of that plane, which then needs
+// only the hat ring. Coordinates are split into index and fraction by adding 2^23 rounding down, on the float adders
+// instead of the conversion unit.
+//
+// Elements whose trace leaves the staged planes (|velocity| dt >= REACH cells) compute with a zero velocity, to keep
+// every index inside the rings, and are evaluated from global memory after the block has met, if any thread has one:
+// one uniform branch per plane instead of two per element.
+//
+// Bound by shared-memory wavefronts (71% of their peak, four in ten of them bank conflicts of lanes whose samples lie in
+// different rows or planes) and instruction issue (65%; about 810 instructions a warp of elements). Measured on B200,
+// velocity advection with the traces formed one after the other, the backward one in its plane's step, against this:
+// 38x48x38 46 and 27 us, 64x96x64 84 and 59 us, 128x192x128 356 and 295 us, 256x384x256 2245 and 1975 us. Planes arrive
+// through registers: 4-byte asynchronous copies took five wavefronts each (2140 us against 2080 us at 256x384x256).
+// Rejected: rows 256 floats apart with a row's four planes side by side, so that rows and planes share banks (2496 us).
+constexpr float TWO23 = 8388608.0f;
+
+// A sample's coordinate: `bits` is its floor plus the constant bits of 2^23 (wrap-around cancels it in an index whose base
+// subtracts SPLIT_BITS), and t its fraction. Coordinates lie in [0, 2^22).
+constexpr int SPLIT_BITS = 0x4B000000;
+struct AxBits {
+  int bits;
+  float t;
+};
+__device__ __forceinline__ AxBits split_bits(float g) {
+  const float x = fmaxf(g, 0.0f);
+  const float shifted = __fadd_rd(x, TWO23);
+  return AxBits{__float_as_int(shifted), x - (shifted - TWO23)};
+}
+
+__device__ __forceinline__ float2 lerp2(float2 a, float2 b, float2 t) {  // lerpm in each lane: b - a as fma(a, -1, b)
+  return __ffma2_rn(t, __ffma2_rn(a, make_float2(-1.0f, -1.0f), b), a);
+}
+
+// The staged planes' float offsets of a sample's lower corner in the planes x and x + 1.
+struct RingAt {
+  int lo, hi;
+};
+template <int PLANE>
+__device__ __forceinline__ RingAt ring_at(int x_bits, int y_bits, int z_bits, int row_base) {
+  const int inplane = y_bits * RZ + z_bits - row_base;  // row_base holds SPLIT_BITS * (RZ + 1)
+  return RingAt{(x_bits & (VR - 1)) * PLANE + inplane, ((x_bits + 1) & (VR - 1)) * PLANE + inplane};
+}
+
+// blend8's operations for two samples at once, of the component whose ring starts at `ring`.
+__device__ __forceinline__ float2 blend_pair(const float* ring, const RingAt& f, const RingAt& b, float2 tx, float2 ty, float2 tz) {
+  auto corner = [&](int at_f, int at_b, int step) { return make_float2(ring[at_f + step], ring[at_b + step]); };
+  const float2 c00 = lerp2(corner(f.lo, b.lo, 0), corner(f.hi, b.hi, 0), tx);
+  const float2 c10 = lerp2(corner(f.lo, b.lo, RZ), corner(f.hi, b.hi, RZ), tx);
+  const float2 c01 = lerp2(corner(f.lo, b.lo, 1), corner(f.hi, b.hi, 1), tx);
+  const float2 c11 = lerp2(corner(f.lo, b.lo, RZ + 1), corner(f.hi, b.hi, RZ + 1), tx);
+  return lerp2(lerp2(c00, c10, ty), lerp2(c01, c11, ty), tz);
+}
+
+__device__ __forceinline__ void ring_corners_at(const float* ring, const RingAt& r, float* a) {
+  a[0] = ring[r.lo];
+  a[1] = ring[r.hi];
+  a[2] = ring[r.lo + RZ];
+  a[3] = ring[r.hi + RZ];
+  a[4] = ring[r.lo + 1];
+  a[5] = ring[r.hi + 1];
+  a[6] = ring[r.lo + RZ + 1];
+  a[7] = ring[r.hi + RZ + 1];
+}
+
+__device__ __forceinline__ F3 zero_unless(bool keep, F3 v) { return f3(keep ? v[0] : 0.0f, keep ? v[1] : 0.0f, keep ? v[2] : 0.0f); }
+
+template <class T, int G, int EPT>
+__device__ __forceinline__ void velocity_march(const Args<T>& A, int seg, float* sm) {
+  const int nx = A.info.dims[0], ny = A.info.dims[1], nz = A.info.dims[2];
+  using M = March<EPT>;
+  constexpr int VRP = M::plane, VHP = M::hat_plane;
+  const Dims gd = group_dims(A.info, G);
+  const int k0 = blockIdx.x * TZ, j0 = blockIdx.y * M::tile;
+  if (j0 >= gd.n1 || k0 >= gd.n2) return;  // a tile past this group's extent (the v and w end rows)
+  const int s = seg * A.seg_len;
+  if (s >= gd.n0) return;
+  const int e = imin_(s + A.seg_len, gd.n0);
+
+  float* vring = sm;                   // [3][VR][VRP]
+  float* hring = vring + 3 * VR * VRP;  // [HR][VHP]
+  const int t = threadIdx.x, ty = t / TZ, tz = t % TZ;
+  const int rowbase = (j0 - 2) * RZ + (k0 - 2), hbase = (j0 - 1) * HZ + (k0 - 1);
+  const int bits_rowbase = (int)((unsigned)rowbase + (unsigned)SPLIT_BITS * (RZ + 1));
+  const int bits_hbase = (int)((unsigned)hbase + (unsigned)SPLIT_BITS * (HZ + 1));
+
+  // staging offsets inside one plane of each component (edge-clamped)
+  int from[3][M::per_thread];
+#pragma unroll
+  for (int n = 0; n < M::per_thread; ++n) {
+    const int el = imin_(t + n * NT, M::staged - 1), r = el / RZ, q = el % RZ;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      from[c][n] = imin_(imax_(j0 - 2 + r, 0), ny + (c == 1) - 1) * (nz + (c == 2)) + imin_(imax_(k0 - 2 + q, 0), nz + (c == 2) - 1);
+  }
+  const Dims vd[3] = {Dims{nx + 1, ny, nz}, Dims{nx, ny + 1, nz}, Dims{nx, ny, nz + 1}};
+  // plane `plane` of the three components: loaded into registers, and later stored into the rings' slot
+  float landing[3][M::per_thread];
+  auto fetch = [&](int plane) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const T* base = A.vel[c] + (size_t)imin_(imax_(plane, 0), vd[c].n0 - 1) * vd[c].n1 * vd[c].n2;
+#pragma unroll
+      for (int n = 0; n < M::per_thread; ++n) landing[c][n] = ldg_f(base + from[c][n]);
+    }
+  };
+  auto land = [&](int plane) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int n = 0; n < M::per_thread; ++n)
+        if (t + n * NT < M::staged) vring[(c * VR + (plane & (VR - 1))) * VRP + t + n * NT] = landing[c][n];
+  };
+
+  // this thread's tile elements (rows j0 + ty + TY n), and its element of the hat plane's ring (t < M::halo)
+  const int tk = k0 + tz, ck = imin_(tk, gd.n2 - 1);
+  int hj, hk;  // position in the hat plane (0..HY-1, 0..HZ-1)
+  if (t < HZ) {
+    hj = 0;
+    hk = t;
+  } else if (t < 2 * HZ) {
+    hj = M::hat_rows - 1;
+    hk = t - HZ;
+  } else if (t < 2 * HZ + M::tile) {
+    hj = 1 + t - 2 * HZ;
+    hk = 0;
+  } else {
+    hj = 1 + t - 2 * HZ - M::tile;
+    hk = HZ - 1;
+  }
+  const bool has_halo = t < M::halo;
+  const int rj = imin_(imax_(j0 - 1 + hj, 0), gd.n1 - 1), rk = imin_(imax_(k0 - 1 + hk, 0), gd.n2 - 1);
+  const int tile_h = (ty + 1) * HZ + (tz + 1), ring_h = hj * HZ + hk;
+  const F3 off = offset_of<G>();
+  const float half = 0.5f * A.dt, reach_dt = fabsf(A.dt);
+
+  // what the correction of a plane needs of this thread's element
+  struct Kept {
+    float lo, hi, hat, data;
+    F3 back;      // the backward sample's index-space coordinates
+    bool global;  // the backward sample is to be taken from global memory
+  };
+
+  // The tile element's hat in plane x (an array plane), and what its correction needs; returns whether its hat is to be
+  // taken from global memory.
+  auto tile_hat = [&](int x, int slot, int n, Kept& kept) -> bool {
+    const int cj = imin_(j0 + ty + n * TY, gd.n1 - 1);
+    const F3 p = add3(f3((float)x, (float)cj, (float)ck), off);
+    const F3 node = ring_node<G, VRP>(vring, x, cj * RZ + ck - rowbase);
+    const bool near = within_reach(node, reach_dt);
+    const F3 vp = zero_unless(near, node);
+    const F3 step = mul3(vp, half);
+    float2 m[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) m[a] = make_float2(p[a] - step[a], p[a] + step[a]);
+    AxBits whole_f[3], whole_b[3], face_f[3], face_b[3];  // at m and at m - 1/2
+    float2 tw[3], tf[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      whole_f[a] = split_bits(m[a].x);
+      whole_b[a] = split_bits(m[a].y);
+      face_f[a] = split_bits(m[a].x - 0.5f);
+      face_b[a] = split_bits(m[a].y - 0.5f);
+      tw[a] = make_float2(whole_f[a].t, whole_b[a].t);
+      tf[a] = make_float2(face_f[a].t, face_b[a].t);
+    }
+    const float2 u = blend_pair(vring, ring_at<VRP>(whole_f[0].bits, face_f[1].bits, face_f[2].bits, bits_rowbase),
+                                ring_at<VRP>(whole_b[0].bits, face_b[1].bits, face_b[2].bits, bits_rowbase), tw[0], tf[1], tf[2]);
+    const float2 v = blend_pair(vring + VR * VRP, ring_at<VRP>(face_f[0].bits, whole_f[1].bits, face_f[2].bits, bits_rowbase),
+                                ring_at<VRP>(face_b[0].bits, whole_b[1].bits, face_b[2].bits, bits_rowbase), tf[0], tw[1], tf[2]);
+    const float2 w = blend_pair(vring + 2 * VR * VRP, ring_at<VRP>(face_f[0].bits, face_f[1].bits, whole_f[2].bits, bits_rowbase),
+                                ring_at<VRP>(face_b[0].bits, face_b[1].bits, whole_b[2].bits, bits_rowbase), tf[0], tf[1], tw[2]);
+    const bool fast = near && within_reach(f3(u.x, v.x, w.x), reach_dt);
+    const bool fast_back = near && within_reach(f3(u.y, v.y, w.y), reach_dt);
+    const F3 src = sub3(p, mul3(zero_unless(fast, f3(u.x, v.x, w.x)), A.dt));
+    kept.back = sub3(sub3(p, mul3(zero_unless(fast_back, f3(u.y, v.y, w.y)), -A.dt)), off);
+    kept.global = !fast_back;
+    kept.data = node[G];  // the component at its own face
+    const F3 g = sub3(src, off);
+    const AxBits gx = split_bits(g[0]), gy = split_bits(g[1]), gz = split_bits(g[2]);
+    float a[8];
+    ring_corners_at(vring + G * VR * VRP, ring_at<VRP>(gx.bits, gy.bits, gz.bits, bits_rowbase), a);
+    kept.hat = blend8(a, gx.t, gy.t, gz.t);
+    range8(a, kept.lo, kept.hi);
+    hring[slot * VHP + tile_h + n * TY * HZ] = kept.hat;
+    return !fast;
+  };
+  // The ring element's hat: the forward trace alone.
+  auto halo_hat = [&](int x, int slot) -> bool {
+    const F3 p = add3(f3((float)x, (float)rj, (float)rk), off);
+    const F3 node = ring_node<G, VRP>(vring, x, rj * RZ + rk - rowbase);
+    const bool near = within_reach(node, reach_dt);
+    const F3 m = sub3(p, mul3(zero_unless(near, node), half));
+    AxBits whole[3], face[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      whole[a] = split_bits(m[a]);
+      face[a] = split_bits(m[a] - 0.5f);
+    }
+    float a[8];
+    ring_corners_at(vring, ring_at<VRP>(whole[0].bits, face[1].bits, face[2].bits, bits_rowbase), a);
+    const float u = blend8(a, whole[0].t, face[1].t, face[2].t);
+    ring_corners_at(vring + VR * VRP, ring_at<VRP>(face[0].bits, whole[1].bits, face[2].bits, bits_rowbase), a);
+    const float v = blend8(a, face[0].t, whole[1].t, face[2].t);
+    ring_corners_at(vring + 2 * VR * VRP, ring_at<VRP>(face[0].bits, face[1].bits, whole[2].bits, bits_rowbase), a);
+    const float w = blend8(a, face[0].t, face[1].t, whole[2].t);
+    const bool fast = near && within_reach(f3(u, v, w), reach_dt);
+    const F3 g = sub3(sub3(p, mul3(zero_unless(fast, f3(u, v, w)), A.dt)), off);
+    const AxBits gx = split_bits(g[0]), gy = split_bits(g[1]), gz = split_bits(g[2]);
+    ring_corners_at(vring + G * VR * VRP, ring_at<VRP>(gx.bits, gy.bits, gz.bits, bits_rowbase), a);
+    hring[slot * VHP + ring_h] = blend8(a, gx.t, gy.t, gz.t);
+    return !fast;
+  };
+  // Hat plane x (clamped to the array) into the ring's slot of x; every thread takes part. Returns, the block having met,
+  // whether some element's backward sample is to be taken from global memory.
+  auto hat_plane = [&](int x, Kept* kept, int arriving) -> bool {
+    const int xc = imin_(imax_(x, 0), gd.n0 - 1), slot = x & (HR - 1);
+    bool slow[EPT], any = false;
+#pragma unroll
+    for (int n = 0; n < EPT; ++n) {
+      slow[n] = tile_hat(xc, slot, n, kept[n]);
+      any = any || slow[n] || kept[n].global;
+    }
+    bool slow_halo = false;
+    if (has_halo) slow_halo = halo_hat(xc, slot);
+    land(arriving);
+    if (!__syncthreads_or(any || slow_halo)) return false;
+    float hat, lo, hi;
+    bool global = false;
+#pragma unroll
+    for (int n = 0; n < EPT; ++n) {
+      global = global || kept[n].global;
+      if (!slow[n]) continue;
+      hat_global<G>(A, xc, imin_(j0 + ty + n * TY, gd.n1 - 1), ck, &hat, &lo, &hi);
+      hring[slot * VHP + tile_h + n * TY * HZ] = hat;
+      kept[n].hat = hat;
+      kept[n].lo = lo;
+      kept[n].hi = hi;
+    }
+    if (slow_halo) {
+      hat_global<G>(A, xc, rj, rk, &hat, &lo, &hi);
+      hring[slot * VHP + ring_h] = hat;
+    }
+    return __syncthreads_or(global);
+  };
+
+  // prologue: planes s-2 .. s+2 of the velocity, hat planes s-1 and s
+#pragma unroll 1
+  for (int p = s - 2; p <= s + 1; ++p) {
+    fetch(p);
+    land(p);
+  }
+  fetch(s + 2);
+  __syncthreads();
+  Kept kept[EPT];
+  hat_plane(s - 1, kept, s + 2);  // below the array: plane 0's hat, as the correction's clamped sample reads it
+  bool global = hat_plane(s, kept, s + 2);
+
+  const size_t plane_stride = (size_t)gd.n1 * gd.n2;
+  T* const next = A.next[G];
+  for (int i = s; i < e; ++i) {
+    // planes i+3 start landing while hat plane i+1 is computed
+    fetch(i + 3);
+    Kept following[EPT];
+    const bool following_global = hat_plane(i + 1, following, i + 3);
+    // the correction (advect.py:34-50, 64): back = hat sampled along the backward trace
+#pragma unroll
+    for (int n = 0; n < EPT; ++n) {
+      const int tj = j0 + ty + n * TY;
+      const AxBits gx = split_bits(kept[n].back[0]), gy = split_bits(kept[n].back[1]), gz = split_bits(kept[n].back[2]);
+      const int gin = gy.bits * HZ + gz.bits - bits_hbase;
+      const float* h0 = hring + (gx.bits & (HR - 1)) * VHP + gin;
+      const float* h1 = hring + ((gx.bits + 1) & (HR - 1)) * VHP + gin;
+      const float a[8] = {h0[0], h1[0], h0[HZ], h1[HZ], h0[1], h1[1], h0[HZ + 1], h1[HZ + 1]};
+      float back = blend8(a, gx.t, gy.t, gz.t);
+      if (global) {
+        float far = back;
+        if (kept[n].global) back_global<G, M::tile, VHP>(A, hring, hbase, j0, k0, i - 1, i, imin_(tj, gd.n1 - 1), ck, &far);
+        back = far;
+      }
+      const float corrected = kept[n].hat + 0.5f * (kept[n].data - back);
+      if (tj < gd.n1 && tk < gd.n2)
+        st_f(next + ((size_t)i * plane_stride + (size_t)tj * gd.n2 + tk), clampf_(corrected, kept[n].lo, kept[n].hi));
+      kept[n] = following[n];
+    }
+    global = following_global;
+  }
+}
+
+// EPT elements per thread and MINB resident blocks per SM: 3 and 1 (80 registers a thread) or 2 and 2 (128).
+template <class T, int EPT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_mac_velocity(const __grid_constant__ Args<T> A) {
+  extern __shared__ float sm[];
+  int z = blockIdx.z;
+  if (z < A.segs[0]) return velocity_march<T, 0, EPT>(A, z, sm);
+  z -= A.segs[0];
+  if (z < A.segs[1]) return velocity_march<T, 1, EPT>(A, z, sm);
+  velocity_march<T, 2, EPT>(A, z - A.segs[1], sm);
+}
+
+// Grids with an axis of 2^22 cells or more, whose coordinates split_bits does not cover.
+template <class T>
+__global__ void __launch_bounds__(NT, 2) k_mac_velocity_long(const __grid_constant__ Args<T> A) {
   extern __shared__ float sm[];
   int z = blockIdx.z;
   if (z < A.segs[0]) return march<T, 0>(A, z, sm);
@@ -602,8 +914,10 @@ __global__ void __launch_bounds__(NT, MINB) k_mac_velocity(Args<T> A) {
   march<T, 2>(A, z - A.segs[1], sm);
 }
 
+// MINB: resident blocks per SM the kernel is compiled for (4 at 256 threads: at most 64 registers a thread;
+// 3: 80; 2: 128).
 template <class T, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_mac_scalars(Args<T> A) {
+__global__ void __launch_bounds__(NT, MINB) k_mac_scalars(const __grid_constant__ Args<T> A) {
   extern __shared__ float sm[];
   march<T, 3>(A, blockIdx.z, sm);
 }
@@ -631,8 +945,7 @@ __global__ void k_segment_lines(const float* __restrict__ seg_sums, int segs, lo
   if (threadIdx.x == 0) partial[f * blocks + blockIdx.x] = slot[0];
 }
 
-constexpr size_t VELOCITY_SMEM = sizeof(float) * (3 * VR * RP + HR * HP);
-constexpr size_t SCALAR_SMEM = sizeof(float) * (3 * VR * RPN + 2 * SR * RPN + 2 * HR * HP);
+constexpr size_t SCALAR_SMEM = sizeof(float) * (3 * VR * RPN + 2 * SR * RPN + 2 * HR * HP + SLACK);
 
 // Segments along x: enough blocks for about six waves of the resident blocks, each segment at least 8 planes.
 static int segments(int n0, long tiles, int groups) {
@@ -647,8 +960,7 @@ static int env_int(const char* name) {
   return v ? atoi(v) : 0;
 }
 
-// Blocks per SM the march kernels run with (PLUME_MAC_BLOCKS = 1 selects the 128-register form).
-// Blocks per SM the marches are compiled for: PLUME_MAC_BLOCKS = 2, 3 or 4 (the default, BLOCKS_PER_SM).
+// Blocks per SM the scalar march is compiled for: PLUME_MAC_BLOCKS = 2, 3 or 4 (the default, BLOCKS_PER_SM).
 static int blocks_per_sm() {
   static const int b = [] {
     const int v = env_int("PLUME_MAC_BLOCKS");
@@ -657,6 +969,48 @@ static int blocks_per_sm() {
   return b;
 }
 
+
+// Elements per thread of the velocity march: two share a tile's halo of hats and its staging between more elements, one
+// leaves more blocks where the grid is small. Measured on B200, two against one: 128x192x128 295 and 305 us,
+// 160x240x160 (bfloat16) 512 and 550 us, 256x384x256 1975 and 2104 us; 80x100x80 98 and 90 us, 64x96x64 70 and 59 us.
+// PLUME_MAC_ELEMENTS = 1, 2 or 3 (k_mac_velocity_long, whatever the axes) overrides the choice, for measurements and to
+// compare the kernels: they give the same floats.
+static int march_elements(const PlumeGridInfo& info) {
+  const int set = env_int("PLUME_MAC_ELEMENTS");
+  if (std::max(info.dims[0], std::max(info.dims[1], info.dims[2])) >= (1 << 22) - 1) return 3;
+  if (set >= 1 && set <= 3) return set;
+  return (long)info.dims[0] * info.dims[1] * info.dims[2] >= 2000000 ? 2 : 1;
+}
+
+// Segments along x of the velocity march, by a cost fitted to measured times: a block of `len` planes takes len + 3 plane
+// times (its prologue forms two more hat planes), each 1.75 + 2.3 w long with w waves of resident blocks sharing the SMs,
+// half of a last wave's missing blocks counted. Measured on B200 with segments of 5 planes against 10 at 38x48x38: 27
+// against 33 us; with 5 segments against 10 at 128x192x128 (one element a thread): 305 against 323 us; with 6 against 5
+// at 160x240x160 (two elements): 512 against 549 us.
+static int velocity_segments(const PlumeGridInfo& info, int ept) {
+  const int set = env_int("PLUME_MAC_VELOCITY_SEGS"), nx = info.dims[0];
+  if (set > 0) return std::min(set, nx);
+  const double resident = 148.0 * (ept == 2 ? 2 : 3);
+  auto tiles = [&](int g) {
+    const int rows = ept * TY;
+    return (double)((info.dims[1] + (g == 1) + rows - 1) / rows) * ((info.dims[2] + (g == 2) + TZ - 1) / TZ);
+  };
+  int best = 1;
+  double least = 0.0;
+  for (int segs = 1; segs <= std::max(1, nx / 4); ++segs) {
+    const int len = (nx + segs - 1) / segs;
+    double blocks = 0.0;
+    for (int g = 0; g < 3; ++g) blocks += tiles(g) * ((nx + (g == 0) + len - 1) / len);
+    double w = blocks / resident;
+    if (w > 1.0) w = 0.5 * (w + std::ceil(w));
+    const double cost = (len + 3.0) * (1.75 + 2.3 * w);
+    if (segs == 1 || cost < least) {
+      best = segs;
+      least = cost;
+    }
+  }
+  return best;
+}
 
 template <class Kernel>
 static int configure(Kernel k, size_t smem, bool& done) {
@@ -686,10 +1040,13 @@ long long mac_partial_floats(const PlumeGridInfo& info) {
 template <class T>
 int launch_mac_velocity(const PlumeGridInfo& info, const T* u, const T* v, const T* w, T* u_next, T* v_next,
                         T* w_next, float dt_over_cell, cudaStream_t st) {
-  static bool configured[5] = {};
-  const int bps = mac::blocks_per_sm();
-  auto kernel = bps == 2 ? mac::k_mac_velocity<T, 2> : (bps == 3 ? mac::k_mac_velocity<T, 3> : mac::k_mac_velocity<T, 4>);
-  int status = mac::configure(kernel, mac::VELOCITY_SMEM, configured[bps]);
+  static bool configured[3] = {};
+  const int form = mac::march_elements(info), ept = form == 2 ? 2 : 1;
+  auto kernel = form == 3 ? mac::k_mac_velocity_long<T>
+                          : (form == 2 ? mac::k_mac_velocity<T, 2, 2> : mac::k_mac_velocity<T, 1, 3>);
+  const size_t smem = ept == 2 ? mac::March<2>::smem : mac::March<1>::smem;
+  const int rows = ept * mac::TY;
+  int status = mac::configure(kernel, smem, configured[form - 1]);
   if (status != PLUME_OK) return status;
   const int nx = info.dims[0], ny = info.dims[1], nz = info.dims[2];
   mac::Args<T> A{};
@@ -701,14 +1058,12 @@ int launch_mac_velocity(const PlumeGridInfo& info, const T* u, const T* v, const
   A.next[1] = v_next;
   A.next[2] = w_next;
   A.dt = dt_over_cell;
-  const int jt = (ny + 1 + mac::TY - 1) / mac::TY, kt = (nz + 1 + mac::TZ - 1) / mac::TZ;
-  int segs = mac::env_int("PLUME_MAC_VELOCITY_SEGS");
-  if (segs <= 0) segs = mac::segments(nx, (long)jt * kt, 3);
-  segs = std::max(1, std::min(segs, nx));
+  const int jt = (ny + 1 + rows - 1) / rows, kt = (nz + 1 + mac::TZ - 1) / mac::TZ;
+  const int segs = mac::velocity_segments(info, ept);
   A.seg_len = (nx + segs - 1) / segs;
   for (int g = 0; g < 3; ++g) A.segs[g] = (nx + (g == 0) + A.seg_len - 1) / A.seg_len;
   const dim3 grid(kt, jt, A.segs[0] + A.segs[1] + A.segs[2]);
-  kernel<<<grid, mac::NT, mac::VELOCITY_SMEM, st>>>(A);
+  kernel<<<grid, mac::NT, smem, st>>>(A);
   return launch_status("fused velocity advection");
 }
 
