@@ -1253,7 +1253,11 @@ static long norm_blocks(const PlumeGridInfo& info) {
 // ---- smoke budget: conserve.py:33-52 + reduce.py:12-38 ------------------------------------------------------
 // Line totals along x in float (reduce.py:12-25); lines added in double in blocks of 256 by a halving tree,
 // then the block partials in order on one thread. The CPU oracle adds in the same order.
-constexpr int SUM_BLOCK = 256;
+//
+// A line's sum is a chain, but its loads are not: LINE_AHEAD of them are under way at a time (one after the other the
+// kernel waited for memory once a plane: the scalar advection phase 38x48x38 31.8 and 29.8 us, 128x192x128 169 and
+// 163 us on B200, a load at a time and so). The tree's last five halvings stay in one warp.
+constexpr int SUM_BLOCK = 256, LINE_AHEAD = 16;
 
 template <class T>
 __global__ void k_line_partials(Dims d, const T* __restrict__ a, const T* __restrict__ b, const T* __restrict__ c,
@@ -1265,16 +1269,27 @@ __global__ void k_line_partials(Dims d, const T* __restrict__ a, const T* __rest
   double value = 0.0;
   if (line < lines) {
     float total = 0.0f;
-    for (int i = 0; i < d.n0; ++i) total = total + ldg_f(src + (long)i * lines + line);
+    const T* from = src + line;
+    for (int i = 0; i < d.n0; i += LINE_AHEAD, from += LINE_AHEAD * lines) {
+      float x[LINE_AHEAD];
+#pragma unroll
+      for (int q = 0; q < LINE_AHEAD; ++q) x[q] = i + q < d.n0 ? ldg_f(from + q * lines) : 0.0f;
+#pragma unroll
+      for (int q = 0; q < LINE_AHEAD; ++q) total = i + q < d.n0 ? total + x[q] : total;
+    }
     value = (double)total;
   }
   slot[threadIdx.x] = value;
   __syncthreads();
-  for (int h = SUM_BLOCK / 2; h >= 1; h >>= 1) {
+  for (int h = SUM_BLOCK / 2; h >= 32; h >>= 1) {
     if ((int)threadIdx.x < h) slot[threadIdx.x] = slot[threadIdx.x] + slot[threadIdx.x + h];
     __syncthreads();
   }
-  if (threadIdx.x == 0) partial[blockIdx.y * blocks + blockIdx.x] = slot[0];
+  if (threadIdx.x >= 32) return;
+  double sum = slot[threadIdx.x];
+#pragma unroll
+  for (int h = 16; h >= 1; h >>= 1) sum = sum + __shfl_down_sync(0xffffffffu, sum, h);
+  if (threadIdx.x == 0) partial[blockIdx.y * blocks + blockIdx.x] = sum;
 }
 
 // totals[0..2] = before, semi-Lagrangian, MacCormack; factor = held / MacCormack (1 when MacCormack <= 0).
