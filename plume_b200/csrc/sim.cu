@@ -594,15 +594,19 @@ __device__ __forceinline__ void face_push_pair(const PlumeGridInfo& info, int i,
   above = __ldg(ff.push[AXIS] + at_hi);
 }
 
-// `below` and `above`: the face's face_push_pair (read only with the confinement push).
-template <int AXIS>
+// `below` and `above`: the face's face_push_pair (read only with the confinement push). The turbulence is none, read from
+// the edges' potentials, or formed in place: a form each, since the lattice hashes of the last, inlined for three axes and
+// four planes, made the other two wait for instructions (2.0 stalls an instruction). Measured on B200 with one form, and
+// so: the forces phase 75x113x91 48 and 44 us, 128x192x128 114 and 97 us, 256x384x256 724 and 632 us.
+enum Turbulence { TURBULENCE_NONE, TURBULENCE_EDGES, TURBULENCE_IN_PLACE };
+template <int AXIS, int TURBULENCE>
 __device__ __forceinline__ float face_forces_value(const PlumeGridInfo& info, float value, int i, int j, int k,
                                                    const FaceForces& ff, float below, float above) {
   if (ff.confinement) {
     float average = 0.5f * (below + above);
     value = value + average * ff.dt;
   }
-  if (ff.turbulence && ff.edge[0]) {
+  if constexpr (TURBULENCE == TURBULENCE_EDGES) {
     constexpr int B = (AXIS + 1) % 3, C = (AXIS + 2) % 3;
     const Dims db{info.dims[0] + (B != 0), info.dims[1] + (B != 1), info.dims[2] + (B != 2)};
     const Dims dc{info.dims[0] + (C != 0), info.dims[1] + (C != 1), info.dims[2] + (C != 2)};
@@ -611,7 +615,7 @@ __device__ __forceinline__ float face_forces_value(const PlumeGridInfo& info, fl
     const float* on_b = ff.edge[B] + at(db, i, j, k);
     const float curl = quotient((__ldg(on_c + sb) - __ldg(on_c)) - (__ldg(on_b + sc) - __ldg(on_b)), ff.inv_to_lattice);
     value = value + ff.strength * curl * ff.dt;
-  } else if (ff.turbulence) {
+  } else if constexpr (TURBULENCE == TURBULENCE_IN_PLACE) {
     const F3 offset = AXIS == 0 ? f3(0.0f, 0.5f, 0.5f) : (AXIS == 1 ? f3(0.5f, 0.0f, 0.5f) : f3(0.5f, 0.5f, 0.0f));
     const F3 face = add3(f3((float)i, (float)j, (float)k), offset);
     constexpr int B = (AXIS + 1) % 3, C = (AXIS + 2) % 3;
@@ -654,7 +658,7 @@ static dim3 face_grid(const PlumeGridInfo& info, int planes) {
 }
 
 // confinement push, turbulence and drag on PLANES faces per thread, every face loaded before any is stored
-template <int AXIS, int PLANES, class T>
+template <int AXIS, int PLANES, int TURBULENCE, class T>
 __device__ __forceinline__ void face_forces_planes(const PlumeGridInfo& info, T* __restrict__ f, int i0, int j, int k,
                                                    const FaceForces& ff) {
   const Dims d = {info.dims[0] + (AXIS == 0), info.dims[1] + (AXIS == 1), info.dims[2] + (AXIS == 2)};
@@ -670,18 +674,18 @@ __device__ __forceinline__ void face_forces_planes(const PlumeGridInfo& info, T*
 #pragma unroll
   for (int p = 0; p < PLANES; ++p)
     if (i0 + p < d.n0)
-      st_f(f + (i0 + p) * plane + at_jk, face_forces_value<AXIS>(info, value[p], i0 + p, j, k, ff, below[p], above[p]));
+      st_f(f + (i0 + p) * plane + at_jk, face_forces_value<AXIS, TURBULENCE>(info, value[p], i0 + p, j, k, ff, below[p], above[p]));
 }
 
-template <class T, int PLANES>
-__global__ void k_face_forces(PlumeGridInfo info, T* __restrict__ u, T* __restrict__ v, T* __restrict__ w,
-                              FaceForces ff) {
+template <class T, int PLANES, int TURBULENCE>
+__global__ void k_face_forces(const __grid_constant__ PlumeGridInfo info, T* __restrict__ u, T* __restrict__ v, T* __restrict__ w,
+                              const __grid_constant__ FaceForces ff) {
   int axis, i0;
   face_planes<PLANES>(info, axis, i0);
   const int j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (axis == 0) face_forces_planes<0, PLANES>(info, u, i0, j, k, ff);
-  else if (axis == 1) face_forces_planes<1, PLANES>(info, v, i0, j, k, ff);
-  else face_forces_planes<2, PLANES>(info, w, i0, j, k, ff);
+  if (axis == 0) face_forces_planes<0, PLANES, TURBULENCE>(info, u, i0, j, k, ff);
+  else if (axis == 1) face_forces_planes<1, PLANES, TURBULENCE>(info, v, i0, j, k, ff);
+  else face_forces_planes<2, PLANES, TURBULENCE>(info, w, i0, j, k, ff);
 }
 
 // Forms the turbulence potentials of `ff` at the edges in `scratch` (`floats` of them) and points `ff` at them, when they fit.
@@ -726,7 +730,9 @@ static int launch_face_forces(const PlumeGridInfo& info, T* u, T* v, T* w, const
                               cudaStream_t st) {
   return with_planes([&](auto P) {
     constexpr int PL = decltype(P)::value;
-    k_face_forces<T, PL><<<face_grid(info, PL), cell_block(), 0, st>>>(info, u, v, w, ff);
+    auto kernel = k_face_forces<T, PL, TURBULENCE_NONE>;
+    if (ff.turbulence) kernel = ff.edge[0] ? k_face_forces<T, PL, TURBULENCE_EDGES> : k_face_forces<T, PL, TURBULENCE_IN_PLACE>;
+    kernel<<<face_grid(info, PL), cell_block(), 0, st>>>(info, u, v, w, ff);
     return launch_status(what);
   });
 }
