@@ -1067,73 +1067,77 @@ __global__ void k_zero_walls(PlumeGridInfo info, T* __restrict__ u, T* __restric
   }
 }
 
-template <class T, int PLANES>
-__global__ void k_divergence(PlumeGridInfo info, const T* __restrict__ u, const T* __restrict__ v,
-                             const T* __restrict__ w, float* __restrict__ div) {  // pressure.py:31-36
+// Streams; every load is issued before the first result, at clamped places instead of behind a branch. Measured on B200,
+// the divergence phase 64x96x64 11.3 and 9.2 us, 256x384x256 91 and 79 us; the gradient, the same way, 38x48x38 8.2 and
+// 6.3 us, 160x240x160 (bfloat16) 69 and 51 us, 256x384x256 172 and 167 us.
+template <class T, int PLANES, bool POW2>
+__global__ void k_divergence(const __grid_constant__ PlumeGridInfo info, Spacing spacing, const T* __restrict__ u,
+                             const T* __restrict__ v, const T* __restrict__ w, float* __restrict__ div) {  // pressure.py:31-36
   const int nx = info.dims[0], ny = info.dims[1], nz = info.dims[2];
   const int i0 = blockIdx.z * PLANES, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= ny || k >= nz) return;
+  float face[PLANES + 1], flux_y[PLANES], flux_z[PLANES];
+#pragma unroll
+  for (int p = 0; p <= PLANES; ++p) face[p] = ldg_f(u + (imin_(i0 + p, nx) * ny + j) * nz + k);
 #pragma unroll
   for (int p = 0; p < PLANES; ++p) {
-    const int i = i0 + p;
-    if (i >= nx) break;
-    float flux = (ldg_f(u + ((i + 1) * ny + j) * nz + k) - ldg_f(u + (i * ny + j) * nz + k)) +
-                 (ldg_f(v + (i * (ny + 1) + j + 1) * nz + k) - ldg_f(v + (i * (ny + 1) + j) * nz + k)) +
-                 (ldg_f(w + (i * ny + j) * (nz + 1) + k + 1) - ldg_f(w + (i * ny + j) * (nz + 1) + k));
-    div[(i * ny + j) * nz + k] = divide(flux, divisor(info.cell_m));
+    const int i = imin_(i0 + p, nx - 1);
+    const T* pv = v + (i * (ny + 1) + j) * nz + k;
+    const T* pw = w + (i * ny + j) * (nz + 1) + k;
+    flux_y[p] = ldg_f(pv + nz) - ldg_f(pv);
+    flux_z[p] = ldg_f(pw + 1) - ldg_f(pw);
   }
+#pragma unroll
+  for (int p = 0; p < PLANES; ++p)
+    if (i0 + p < nx)
+      div[((i0 + p) * ny + j) * nz + k] = per_span<POW2>((face[p + 1] - face[p]) + flux_y[p] + flux_z[p], 1, spacing);
 }
 
 // subtract_gradient_kernel (pressure.py:95-116) over the three face arrays (blockIdx.z segments).
-// The face's pressure difference (q_above - q_below); false for a closed wall face, which is left alone.
+// The face's pressures on both sides (0 beyond an open wall), without a branch; false for a closed wall face, which is
+// left alone.
 template <int AXIS>
 __device__ __forceinline__ bool gradient_at(const PlumeGridInfo& info, const float* __restrict__ q, int i, int j, int k,
                                             float& q_above, float& q_below) {
   const Dims d = dims_of(info);
-  const int index = AXIS == 0 ? i : (AXIS == 1 ? j : k);
-  const int below = AXIS == 0 ? at(d, i - 1, j, k) : (AXIS == 1 ? at(d, i, j - 1, k) : at(d, i, j, k - 1));
-  q_above = 0.0f;
-  q_below = 0.0f;
-  if (index == 0) {
-    if (info.open_lo[AXIS] == 0) return false;
-    q_above = __ldg(q + at(d, i, j, k));
-  } else if (index == info.dims[AXIS]) {
-    if (info.open_hi[AXIS] == 0) return false;
-    q_below = __ldg(q + below);
-  } else {
-    q_above = __ldg(q + at(d, i, j, k));
-    q_below = __ldg(q + below);
-  }
-  return true;
+  const int index = AXIS == 0 ? i : (AXIS == 1 ? j : k), n = info.dims[AXIS];
+  const int stride = AXIS == 0 ? d.n1 * d.n2 : (AXIS == 1 ? d.n2 : 1), here = at(d, i, j, k);
+  const bool first = index == 0, last = index == n;
+  const float above = __ldg(q + (last ? here - stride : here)), below = __ldg(q + (first ? here : here - stride));
+  q_above = last ? 0.0f : above;
+  q_below = first ? 0.0f : below;
+  return !(first && info.open_lo[AXIS] == 0) && !(last && info.open_hi[AXIS] == 0);
 }
 
-template <int AXIS, int PLANES, class T>
-__device__ __forceinline__ void subtract_gradient_planes(const PlumeGridInfo& info, T* __restrict__ f,
+template <int AXIS, int PLANES, bool POW2, class T>
+__device__ __forceinline__ void subtract_gradient_planes(const PlumeGridInfo& info, const Spacing& spacing, T* __restrict__ f,
                                                          const float* __restrict__ q, int i0, int j, int k) {
   const Dims d = {info.dims[0] + (AXIS == 0), info.dims[1] + (AXIS == 1), info.dims[2] + (AXIS == 2)};
   if (j >= d.n1 || k >= d.n2) return;
-  const long plane = (long)d.n1 * d.n2, at_jk = (long)j * d.n2 + k;
+  const int plane = d.n1 * d.n2;
+  T* const from = f + (j * d.n2 + k);
   float value[PLANES], above[PLANES], below[PLANES];
   bool apply[PLANES];
 #pragma unroll
   for (int p = 0; p < PLANES; ++p) {
-    apply[p] = i0 + p < d.n0 && gradient_at<AXIS>(info, q, i0 + p, j, k, above[p], below[p]);
-    if (apply[p]) value[p] = ld_f(f + (i0 + p) * plane + at_jk);
+    const int i = imin_(i0 + p, d.n0 - 1);
+    apply[p] = gradient_at<AXIS>(info, q, i, j, k, above[p], below[p]) && i0 + p < d.n0;
+    value[p] = ld_f(from + i * plane);
   }
 #pragma unroll
   for (int p = 0; p < PLANES; ++p)
-    if (apply[p]) st_f(f + (i0 + p) * plane + at_jk, value[p] - divide(above[p] - below[p], divisor(info.cell_m)));
+    if (apply[p]) st_f(from + (i0 + p) * plane, value[p] - per_span<POW2>(above[p] - below[p], 1, spacing));
 }
 
-template <class T, int PLANES>
-__global__ void k_subtract_gradient(PlumeGridInfo info, T* __restrict__ u, T* __restrict__ v, T* __restrict__ w,
-                                    const float* __restrict__ q) {
+template <class T, int PLANES, bool POW2>
+__global__ void k_subtract_gradient(const __grid_constant__ PlumeGridInfo info, Spacing spacing, T* __restrict__ u,
+                                    T* __restrict__ v, T* __restrict__ w, const float* __restrict__ q) {
   int axis, i0;
   face_planes<PLANES>(info, axis, i0);
   const int j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (axis == 0) subtract_gradient_planes<0, PLANES>(info, u, q, i0, j, k);
-  else if (axis == 1) subtract_gradient_planes<1, PLANES>(info, v, q, i0, j, k);
-  else subtract_gradient_planes<2, PLANES>(info, w, q, i0, j, k);
+  if (axis == 0) subtract_gradient_planes<0, PLANES, POW2>(info, spacing, u, q, i0, j, k);
+  else if (axis == 1) subtract_gradient_planes<1, PLANES, POW2>(info, spacing, v, q, i0, j, k);
+  else subtract_gradient_planes<2, PLANES, POW2>(info, spacing, w, q, i0, j, k);
 }
 
 template <class T>
@@ -1141,9 +1145,11 @@ static int launch_divergence(const PlumeGridInfo& info, const T* u, const T* v, 
                              cudaStream_t st) {
   return with_planes([&](auto P) {
     constexpr int PL = decltype(P)::value;
-    k_divergence<T, PL><<<cell_grid_planes(info.dims[0], info.dims[1], info.dims[2], PL), cell_block(), 0, st>>>(
-        info, u, v, w, div);
-    return launch_status("divergence");
+    return with_spacing(info.cell_m, [&](auto pow2, Spacing spacing) {
+      k_divergence<T, PL, decltype(pow2)::value>
+          <<<cell_grid_planes(info.dims[0], info.dims[1], info.dims[2], PL), cell_block(), 0, st>>>(info, spacing, u, v, w, div);
+      return launch_status("divergence");
+    });
   });
 }
 
@@ -1151,8 +1157,10 @@ template <class T>
 static int launch_subtract_gradient(const PlumeGridInfo& info, T* u, T* v, T* w, const float* q, cudaStream_t st) {
   return with_planes([&](auto P) {
     constexpr int PL = decltype(P)::value;
-    k_subtract_gradient<T, PL><<<face_grid(info, PL), cell_block(), 0, st>>>(info, u, v, w, q);
-    return launch_status("subtract gradient");
+    return with_spacing(info.cell_m, [&](auto pow2, Spacing spacing) {
+      k_subtract_gradient<T, PL, decltype(pow2)::value><<<face_grid(info, PL), cell_block(), 0, st>>>(info, spacing, u, v, w, q);
+      return launch_status("subtract gradient");
+    });
   });
 }
 
