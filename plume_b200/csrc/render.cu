@@ -78,8 +78,8 @@ __device__ __forceinline__ int past_brick(int s, int end, float count) {
 // A warp takes seven bricks of a row along z: 29 columns of cells, 5 x 5 loads each along the rows, then the columns of
 // each brick. A thread per brick read its 125 cells one row of five after the other, each lane on another cache line.
 constexpr int ROW_BRICKS = 7, ROW_WARPS = 4;
-static dim3 brick_row_grid(const Dims& b) {
-  return dim3((b.n2 + ROW_BRICKS - 1) / ROW_BRICKS, (b.n1 + ROW_WARPS - 1) / ROW_WARPS, b.n0);
+static dim3 brick_row_grid(const Dims& b) {  // tiles of (j, k) along x, which has room for any axis
+  return dim3((unsigned)((b.n2 + ROW_BRICKS - 1) / ROW_BRICKS) * ((b.n1 + ROW_WARPS - 1) / ROW_WARPS), 1, b.n0);
 }
 struct BrickRow {
   int i, j, k;  // the first cell on each axis, k this lane's column
@@ -87,11 +87,12 @@ struct BrickRow {
 };
 __device__ __forceinline__ bool brick_row(const Dims& d, BrickRow& r) {
   const Dims b = brick_dims(d);
-  const int bi = blockIdx.z, bj = blockIdx.y * ROW_WARPS + threadIdx.y, bk = blockIdx.x * ROW_BRICKS + threadIdx.x / BRICK;
+  const unsigned across = (b.n2 + ROW_BRICKS - 1) / ROW_BRICKS, tile_j = blockIdx.x / across, tile_k = blockIdx.x - tile_j * across;
+  const int bi = blockIdx.z, bj = tile_j * ROW_WARPS + threadIdx.y, bk = tile_k * ROW_BRICKS + threadIdx.x / BRICK;
   if (bj >= b.n1) return false;
   r.i = bi * BRICK;
   r.j = bj * BRICK;
-  r.k = imin_(blockIdx.x * ROW_BRICKS * BRICK + threadIdx.x, d.n2 - 1);
+  r.k = imin_(tile_k * ROW_BRICKS * BRICK + threadIdx.x, d.n2 - 1);
   r.brick = threadIdx.x % BRICK == 0 && threadIdx.x < ROW_BRICKS * BRICK && bk < b.n2 ? at(b, bi, bj, bk) : -1;
   return true;
 }
@@ -368,7 +369,8 @@ __global__ void __launch_bounds__(32 * LIGHT_ROWS, 4) k_light_volume(Dims d, con
   __shared__ unsigned short queue[LIGHT_ROWS * 32];
   __shared__ int queued;
   const int lane = threadIdx.x, warp = threadIdx.y;
-  const int i = blockIdx.z, k = blockIdx.x * 32 + lane, j0 = blockIdx.y * LIGHT_ROWS;
+  const unsigned across = (d.n2 + 31) / 32, tile_j = blockIdx.x / across, tile_k = blockIdx.x - tile_j * across;
+  const int i = blockIdx.z, k0 = tile_k * 32, k = k0 + lane, j0 = tile_j * LIGHT_ROWS;
   if (lane == 0 && warp == 0) queued = 0;
   __syncthreads();
   if (j0 + warp < d.n1) {
@@ -389,7 +391,7 @@ __global__ void __launch_bounds__(32 * LIGHT_ROWS, 4) k_light_volume(Dims d, con
   const int count = queued;
 #pragma unroll 1
   for (int b = warp * 32 + lane; b < count; b += 32 * LIGHT_ROWS) {
-    const int e = queue[b], j = j0 + e / 32, kk = blockIdx.x * 32 + e % 32;
+    const int e = queue[b], j = j0 + e / 32, kk = k0 + e % 32;
     light[at(d, i, j, kk)] = light_at(d, smoke, toward, cell_m, opacity, bricks, i, j, kk);
   }
 }
@@ -708,7 +710,7 @@ static int light_volume(const Dims& d, const T* smoke, F3 toward, float cell_m, 
     int status = launch_status("smoke brick map");
     if (status != PLUME_OK || (status = brick_reach(b, map, bricks, st)) != PLUME_OK) return status;
   }
-  const dim3 grid((d.n2 + 31) / 32, (d.n1 + LIGHT_ROWS - 1) / (LIGHT_ROWS), d.n0);
+  const dim3 grid((unsigned)((d.n2 + 31) / 32) * ((d.n1 + LIGHT_ROWS - 1) / LIGHT_ROWS), 1, d.n0);
   k_light_volume<T><<<grid, dim3(32, LIGHT_ROWS), 0, st>>>(d, smoke, toward, cell_m, opacity, light, bricks, march_cells);
   return launch_status("light volume");
 }

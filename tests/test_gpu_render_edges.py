@@ -72,3 +72,13 @@ def test_gradient(cuda_device, cells, blur_cells):
                                RenderSettings(normal_blur_cells=blur_cells), cells, NORMAL_LAYOUT)
     renderer.prepare(smoke, 0.05)
     assert_same(host(gradient), renderer.gradient, "gradient")
+
+
+def test_light_of_a_long_second_axis(cuda_device):
+    """More rows than a launch has blocks along its second axis."""
+    smoke = torch.from_numpy(sparse((1, 2048, 3))).to("cuda:0").repeat(1, 300, 1).contiguous()
+    light = host(LightVolume(tuple(smoke.shape), (0.0, 0.0, 1.0), 1.0, "cuda:0").compute(smoke, 0.05, march_cells=True))
+    part = smoke[:, :4096].contiguous()
+    expected = host(LightVolume(tuple(part.shape), (0.0, 0.0, 1.0), 1.0, "cuda:0").compute(part, 0.05, march_cells=True))
+    assert_same(light[:, :4095], expected[:, :4095], "first rows")  # the part's last row has no neighbour beyond it
+    assert_same(light[:, -2048:-1], expected[:, 2048:4095], "last rows")
