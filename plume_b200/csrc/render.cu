@@ -4,6 +4,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "light_range.cuh"
 
 namespace plume {
 
@@ -237,14 +238,6 @@ __device__ __forceinline__ SplitAxis split_axis(float g, int n) {
   return SplitAxis{__float_as_uint(shifted), x - (shifted - TWO23)};
 }
 
-// How many steps of `delta` from the cell `corner` stay in [0, n - 1) by more than `margin` cells, possibly negative; none
-// when delta is no number, or so small that a sample's side of 0 is a matter of rounding.
-__device__ __forceinline__ float samples_inside(float delta, float corner, int n, float margin) {
-  const float last = (float)(n - 1);
-  if (!(fabsf(delta) > 1.0e-12f)) return fabsf(delta) <= 1.0e-12f && corner >= 1.0f && corner < last ? 3.0e38f : 0.0f;
-  return ((delta > 0.0f ? last - corner : corner) - margin) / fabsf(delta);
-}
-
 // The column of one cell's march when an extent or the sample count passes SPLIT_LIMIT: every sample, indices converted.
 template <class T>
 __device__ __noinline__ float column_long(const Dims& d, const T* __restrict__ smoke, F3 toward, F3 corner, int steps, float step) {
@@ -277,7 +270,7 @@ __device__ __forceinline__ float light_at(const Dims& d, const T* __restrict__ s
     if (imax_(widest, steps) >= SPLIT_LIMIT) return exp_f(-opacity * column_long(d, smoke, toward, corner, steps, step) * cell_m);
     // the computed points (i, j, k) + toward * ((s + 0.5) * step), from the cell's lower corner, are within
     // (2 * length + 2 * extent) * 2^-24 cells of the exact line
-    const float margin = (4.0f * length + 4.0f * (float)(widest + 1)) * 5.9604645e-8f + 1.0e-3f;
+    const float margin = march_margin(length, widest);
     const SkipAxis skip_x = skip_axis(toward[0] * step, d.n0), skip_y = skip_axis(toward[1] * step, d.n1),
                    skip_z = skip_axis(toward[2] * step, d.n2);
     const Dims bd = brick_dims(d);
@@ -304,7 +297,7 @@ __device__ __forceinline__ float light_at(const Dims& d, const T* __restrict__ s
     const float inner = fminf(fminf(samples_inside(toward[0] * step, corner[0], d.n0, margin),
                                     samples_inside(toward[1] * step, corner[1], d.n1, margin)),
                               samples_inside(toward[2] * step, corner[2], d.n2, margin));
-    const float to = fminf(floorf(inner) - 1.0f, end) - (float)(LIGHT_RUN - 1);
+    const float to = last_run(inner, end, LIGHT_RUN);
     float s = 0.0f;
     // runs of LIGHT_RUN samples whose corners lie in the array; only the first looks its brick up
     while (s <= to) {
