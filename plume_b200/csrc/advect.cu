@@ -34,6 +34,7 @@
 #include <cstdlib>
 
 #include "advect.cuh"
+#include "march_plan.cuh"
 
 namespace plume {
 namespace mac {
@@ -903,7 +904,8 @@ __global__ void __launch_bounds__(NT, MINB) k_mac_velocity(const __grid_constant
   velocity_march<T, 2, EPT>(A, z - A.segs[1], sm);
 }
 
-// Grids with an axis of 2^22 cells or more, whose coordinates split_bits does not cover.
+// Grids with an axis of 2^22 cells or more, whose coordinates split_bits does not cover, and time steps that are not finite
+// (march_form).
 template <class T>
 __global__ void __launch_bounds__(NT, 2) k_mac_velocity_long(const __grid_constant__ Args<T> A) {
   extern __shared__ float sm[];
@@ -970,18 +972,6 @@ static int blocks_per_sm() {
 }
 
 
-// Elements per thread of the velocity march: two share a tile's halo of hats and its staging between more elements, one
-// leaves more blocks where the grid is small. Measured on B200, two against one: 128x192x128 295 and 305 us,
-// 160x240x160 (bfloat16) 512 and 550 us, 256x384x256 1975 and 2104 us; 80x100x80 98 and 90 us, 64x96x64 70 and 59 us.
-// PLUME_MAC_ELEMENTS = 1, 2 or 3 (k_mac_velocity_long, whatever the axes) overrides the choice, for measurements and to
-// compare the kernels: they give the same floats.
-static int march_elements(const PlumeGridInfo& info) {
-  const int set = env_int("PLUME_MAC_ELEMENTS");
-  if (std::max(info.dims[0], std::max(info.dims[1], info.dims[2])) >= (1 << 22) - 1) return 3;
-  if (set >= 1 && set <= 3) return set;
-  return (long)info.dims[0] * info.dims[1] * info.dims[2] >= 2000000 ? 2 : 1;
-}
-
 // Segments along x of the velocity march, by a cost fitted to measured times: a block of `len` planes takes len + 3 plane
 // times (its prologue forms two more hat planes), each 1.75 + 2.3 w long with w waves of resident blocks sharing the SMs,
 // half of a last wave's missing blocks counted. Measured on B200 with segments of 5 planes against 10 at 38x48x38: 27
@@ -1041,7 +1031,7 @@ template <class T>
 int launch_mac_velocity(const PlumeGridInfo& info, const T* u, const T* v, const T* w, T* u_next, T* v_next,
                         T* w_next, float dt_over_cell, cudaStream_t st) {
   static bool configured[3] = {};
-  const int form = mac::march_elements(info), ept = form == 2 ? 2 : 1;
+  const int form = mac::march_form(info.dims, dt_over_cell, mac::env_int("PLUME_MAC_ELEMENTS")), ept = form == 2 ? 2 : 1;
   auto kernel = form == 3 ? mac::k_mac_velocity_long<T>
                           : (form == 2 ? mac::k_mac_velocity<T, 2, 2> : mac::k_mac_velocity<T, 1, 3>);
   const size_t smem = ept == 2 ? mac::March<2>::smem : mac::March<1>::smem;
