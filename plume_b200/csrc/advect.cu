@@ -30,7 +30,6 @@
 // each line in order and the lines in double. Temperature's dissipation (dissipate.py:10-15) is applied as
 // it is stored.
 #include <algorithm>
-#include <cmath>
 #include <cstdlib>
 
 #include "advect.cuh"
@@ -972,36 +971,6 @@ static int blocks_per_sm() {
 }
 
 
-// Segments along x of the velocity march, by a cost fitted to measured times: a block of `len` planes takes len + 3 plane
-// times (its prologue forms two more hat planes), each 1.75 + 2.3 w long with w waves of resident blocks sharing the SMs,
-// half of a last wave's missing blocks counted. Measured on B200 with segments of 5 planes against 10 at 38x48x38: 27
-// against 33 us; with 5 segments against 10 at 128x192x128 (one element a thread): 305 against 323 us; with 6 against 5
-// at 160x240x160 (two elements): 512 against 549 us.
-static int velocity_segments(const PlumeGridInfo& info, int ept) {
-  const int set = env_int("PLUME_MAC_VELOCITY_SEGS"), nx = info.dims[0];
-  if (set > 0) return std::min(set, nx);
-  const double resident = 148.0 * (ept == 2 ? 2 : 3);
-  auto tiles = [&](int g) {
-    const int rows = ept * TY;
-    return (double)((info.dims[1] + (g == 1) + rows - 1) / rows) * ((info.dims[2] + (g == 2) + TZ - 1) / TZ);
-  };
-  int best = 1;
-  double least = 0.0;
-  for (int segs = 1; segs <= std::max(1, nx / 4); ++segs) {
-    const int len = (nx + segs - 1) / segs;
-    double blocks = 0.0;
-    for (int g = 0; g < 3; ++g) blocks += tiles(g) * ((nx + (g == 0) + len - 1) / len);
-    double w = blocks / resident;
-    if (w > 1.0) w = 0.5 * (w + std::ceil(w));
-    const double cost = (len + 3.0) * (1.75 + 2.3 * w);
-    if (segs == 1 || cost < least) {
-      best = segs;
-      least = cost;
-    }
-  }
-  return best;
-}
-
 template <class Kernel>
 static int configure(Kernel k, size_t smem, bool& done) {
   if (done) return PLUME_OK;
@@ -1049,7 +1018,7 @@ int launch_mac_velocity(const PlumeGridInfo& info, const T* u, const T* v, const
   A.next[2] = w_next;
   A.dt = dt_over_cell;
   const int jt = (ny + 1 + rows - 1) / rows, kt = (nz + 1 + mac::TZ - 1) / mac::TZ;
-  const int segs = mac::velocity_segments(info, ept);
+  const int segs = mac::march_segments(info.dims, ept, mac::TY, mac::TZ, mac::env_int("PLUME_MAC_VELOCITY_SEGS"));
   A.seg_len = (nx + segs - 1) / segs;
   for (int g = 0; g < 3; ++g) A.segs[g] = (nx + (g == 0) + A.seg_len - 1) / A.seg_len;
   const dim3 grid(kt, jt, A.segs[0] + A.segs[1] + A.segs[2]);
