@@ -487,8 +487,10 @@ __device__ __forceinline__ F3 sample_vec(const float* __restrict__ f, const Dims
 // The camera march's brick map: over each brick and the next cell past it on each axis (every corner a sample
 // with lower corner in the brick can blend), 2 when some smoke is > 0, plus 1 when the temperature may glow. The
 // temperature cannot glow when its largest value is below glow_start by more than the rounding of three lerps (16
-// ulps), or when it is one value <= glow_start: a blend of equal corners is exactly that value. A sample in a brick
-// without smoke has alpha 0, one where nothing glows glow 0; where neither holds it adds exactly nothing.
+// ulps). A sample in a brick without smoke has alpha 0, one where nothing glows glow 0; where neither holds it adds
+// nothing. Outside the smoke a temperature of one value <= glow_start does not glow either: its blends are that value to
+// a few ulps (exactly, for 0 and powers of two), and ulps above glow_start, which the blends of some other values have
+// at a sample in fifty, are not taken for glow there. Within the smoke they are, as they are without the map.
 template <class T>
 __global__ void __launch_bounds__(32 * ROW_WARPS) k_march_bricks(Dims d, const T* __restrict__ smoke, const T* __restrict__ temperature,
                                                                  float glow_start, float* __restrict__ bricks) {
@@ -509,8 +511,9 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) k_march_bricks(Dims d, const T
   most = over_columns(most, larger);
   hot = over_columns(hot, larger);
   cold = over_columns(cold, [](float x, float y) { return fminf(x, y); });
-  const bool dark = (hot + fabsf(hot) * 9.5367432e-7f < glow_start) || (cold == hot && hot <= glow_start);
-  if (r.brick >= 0) bricks[r.brick] = (most > 0.0f ? 2.0f : 0.0f) + (dark ? 0.0f : 1.0f);
+  const bool smoky = most > 0.0f;
+  const bool dark = (hot + fabsf(hot) * 9.5367432e-7f < glow_start) || (!smoky && cold == hot && hot <= glow_start);
+  if (r.brick >= 0) bricks[r.brick] = (smoky ? 2.0f : 0.0f) + (dark ? 0.0f : 1.0f);
 }
 
 // sample_index_space from its axes; p: the lower corner.
