@@ -213,10 +213,13 @@ class FlowFit:
     in the backward walk), else from zero. Either way the gradient is that of the exact projection, to within
     the residual the solves leave.
 
-    Tape: a substep's record is 12 face arrays (15 with confinement) and 5 cell arrays. The forward pass of loss_and_grad keeps the
-    records of the last segments whole while they fit `tape_bytes` (by default half the device memory free when
-    the gradient is asked for, or what the caching allocator holds idle when that is enough for every record), and
-    the backward pass recomputes only the segments it did not keep. The forward is deterministic, so a kept record and a recomputed one are the same floats, and the budget changes the
+    Tape: a substep's record is 12 face arrays (15 with confinement) and 5 cell arrays. The forward pass of loss_and_grad keeps
+    the records of the last segments whole while they fit `tape_bytes`, and the backward pass recomputes only the segments
+    it did not keep. The default budget is half the device memory free when the gradient is asked for, or what the caching
+    allocator holds idle when that is enough for every record. Idle memory may turn out not to serve (blocks too small, or
+    of another stream): as soon as the allocator takes more from the driver for a record, the tape is cut back to the first
+    budget, and when memory runs out with a tape in idle memory the gradient is formed again under it. The
+    forward is deterministic, so a kept record and a recomputed one are the same floats, and the budget changes the
     time, not the gradient."""
 
     def __init__(self, recipe, source_shape, corner, substeps: int, device: str = "cuda:0", window=(0.0, math.inf),
@@ -342,10 +345,12 @@ class FlowFit:
                    ambient, N.stream())
         return rec
 
-    def forward(self, source: torch.Tensor, taped_from: int | None = None):
+    def forward(self, source: torch.Tensor, taped_from: int | None = None, reserved: int | None = None):
         """The run from rest with the source; returns the checkpoints (one full state every checkpoint_every
         substeps) and leaves the final state in the work grid. With `taped_from`, also returns the records of
-        substeps taped_from.. (a dict by substep)."""
+        substeps taped_from.. (a dict by substep). `reserved`: the records are to come from the allocator's idle
+        memory, of which it had this much with what is in use; when it takes more, the records kept are those of
+        the driver's budget, whole segments from the end."""
         g = self.grid
         for x in (*g.velocity_fields(), g.smoke):
             x.data.zero_()
@@ -359,6 +364,11 @@ class FlowFit:
             rec = self._substep(n, source, record=taped)
             if taped:
                 records[n] = rec
+                if reserved is not None and torch.cuda.memory_reserved(torch.device(self.device)) > reserved:
+                    reserved = None
+                    taped_from = max(taped_from, self._kept_within(self._driver_budget()))
+                    records = {m: kept for m, kept in records.items() if m >= taped_from}
+            del rec
         return (checkpoints, records) if taped_from is not None else checkpoints
 
     def record_bytes(self) -> int:
@@ -367,25 +377,34 @@ class FlowFit:
         faces = sum(x.data.numel() for x in g.velocity_fields())
         return 4 * ((5 if self.confined else 4) * faces + 5 * g.smoke.data.numel()) + 8 * 3
 
-    def _taped_from(self) -> int:
-        """The first substep whose record the forward keeps: whole segments from the end, within the budget."""
-        budget = self.tape_bytes
-        if budget is None:
-            # The driver is asked only when the whole tape does not fit the memory that the caching allocator holds
-            # idle: the query waits for the driver's locks. Measured on a B200 host shared with other programs, a
-            # gradient at 96 x 144 x 96 over 4 substeps: 11.8 ms without it; with it 12.3 ms at the median and 17 to
-            # 22 ms on average (a fifth to a third of the calls took 3 to 90 ms).
-            device = torch.device(self.device)
-            idle = torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
-            if self.substeps * self.record_bytes() <= idle:
-                return 0
-            free, _ = torch.cuda.mem_get_info(device)
-            budget = free // 2
-        keep = int(budget // self.record_bytes())
-        first = self.substeps - keep
+    def _kept_within(self, budget: int) -> int:
+        """The first substep whose record fits the budget: whole segments from the end."""
+        first = self.substeps - int(budget // self.record_bytes())
         if first <= 0:
             return 0
         return min(self.substeps, -(-first // self.every) * self.every)
+
+    def _driver_budget(self) -> int:
+        free, _ = torch.cuda.mem_get_info(torch.device(self.device))
+        return free // 2
+
+    def _plan_tape(self):
+        """The first substep whose record the forward is to keep, and, when the records are to come from what the
+        allocator holds idle, its reserved bytes (else None)."""
+        if self.tape_bytes is not None:
+            return self._kept_within(self.tape_bytes), None
+        # The driver is asked only when the whole tape does not fit the memory that the caching allocator holds
+        # idle: the query waits for the driver's locks. Measured on a B200 host shared with other programs, a
+        # gradient at 96 x 144 x 96 over 4 substeps: 11.8 ms without it; with it 12.3 ms at the median and 17 to
+        # 22 ms on average (a fifth to a third of the calls took 3 to 90 ms).
+        device = torch.device(self.device)
+        reserved = torch.cuda.memory_reserved(device)
+        if self.substeps * self.record_bytes() <= reserved - torch.cuda.memory_allocated(device):
+            return 0, reserved
+        return self._kept_within(self._driver_budget()), None
+
+    def _taped_from(self) -> int:
+        return self._plan_tape()[0]
 
     def _thickness(self, target):
         g = self.grid
@@ -487,8 +506,17 @@ class FlowFit:
         final thickness); the confinement strength's derivative when the recipe applies confinement."""
         source = source.to(self.device, torch.float32).contiguous()
         target = target.to(self.device, torch.float32).contiguous()
-        taped_from = self._taped_from()
-        checkpoints, taped = self.forward(source, taped_from)
+        taped_from, reserved = self._plan_tape()
+        try:
+            return self._loss_and_grad(source, target, taped_from, reserved)
+        except torch.OutOfMemoryError:
+            if reserved is None:
+                raise
+        # idle memory held the tape, but the rest of the pass found none; the first attempt's is free again here
+        return self._loss_and_grad(source, target, self._kept_within(self._driver_budget()), None)
+
+    def _loss_and_grad(self, source, target, taped_from: int, reserved: int | None):
+        checkpoints, taped = self.forward(source, taped_from, reserved)
         loss, thickness, a_smoke = self._thickness(target)
         g = self.grid
         self.adjoint_grid.pressure.zero_()
@@ -499,7 +527,7 @@ class FlowFit:
         for segment in reversed(range(len(checkpoints))):
             first = segment * self.every
             last = min(first + self.every, self.substeps)
-            if first >= taped_from:
+            if first in taped:
                 records = [taped.pop(n) for n in range(first, last)]
             else:
                 self._load(checkpoints[segment])
