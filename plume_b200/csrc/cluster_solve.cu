@@ -77,7 +77,8 @@ struct ClusterArgs {
 extern __shared__ __align__(16) float smem[];
 
 // 1 / d for quotient(): two Newton steps in double from the approximate float reciprocal (relative error 2^-23, then
-// 2^-46, then the double's rounding), without a division's branch.
+// 2^-46, then the double's rounding), without a division's branch. For divisors the approximate one holds for
+// (spacing_in_range).
 __device__ __forceinline__ double reciprocal(float d) {
   const double x = (double)d;
   double y = (double)__fdividef(1.0f, d);
@@ -753,9 +754,18 @@ int prepare_cluster_solve() {
   return PLUME_OK;
 }
 
+// Whether reciprocal() holds for a level: the approximate division it starts from does for divisors of 2^-126 to 2^126,
+// which the coupling sums are in always, cell_volume * cell_m * cell_m for spacings of about 1e-19 to 9e18 m.
+static bool spacing_in_range(const PlumeGridInfo& info) {
+  const float h2 = info.cell_m * info.cell_m;
+  return h2 <= 0x1p126f && info.fill_hi[0] * info.fill_hi[1] * info.fill_hi[2] * info.cell_m * info.cell_m >= 0x1p-126f;
+}
+
 bool cluster_solve_runs(const ClusterSolve& s) {
   int device = 0;
   if (s.count < 1 || s.count > CLUSTER_MAX_LEVELS || cluster_solve_bytes(s) > CS_MAX_SMEM) return false;
+  for (int l = 0; l < s.count; ++l)
+    if (!spacing_in_range(s.levels[l].info)) return false;
   if (s.single_from < s.count && !cluster_solve_single(s.levels[s.single_from].info)) return false;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return false;
   return s.ctas <= 8 || g_cluster_16[device];
