@@ -41,16 +41,16 @@ PHASE_BYTES = {"forces": 32.0, "velocity advection": 24.0, "divergence": 16.0, "
                "gradient": 28.0, "scalar advection": 44.0}
 MG_BYTES_PER_CYCLE = 74.0
 # DRAM bytes (read + write) per top-level cell per V-cycle that ncu counted for the pressure-solve kernels of
-# the 128x192x128 step (965.7 MB per substep at 4 cycles, every level in the natural layout); the solve's
-# traffic scales with the level cells.
-MG_TRAFFIC_PER_CYCLE = 965.7e6 / (128 * 192 * 128) / 4
+# the 128x192x128 step (1084.4 MB per substep at 4 cycles, every level in the natural layout, caches flushed before each
+# launch); the solve's traffic scales with the level cells.
+MG_TRAFFIC_PER_CYCLE = 1084.4e6 / (128 * 192 * 128) / 4
 # A top level in colour-split storage (levels of at least plume_split_min_cells cells), per top-level cell,
 # from one ncu capture of each kernel at 256x384x256 (dram__bytes_read.sum + dram__bytes_write.sum): a colour
-# pass 175.9 MB, the residual and restriction 219.3 MB, the prolongation 158.1 MB per V-cycle (8 passes per
+# pass 173.9 MB, the residual and restriction 225.8 MB, the prolongation 153.0 MB per V-cycle (8 passes per
 # cycle at 2 + 2 sweeps); the three layout conversions 461.5 MB per solve. The levels below it are a natural
 # hierarchy of one eighth the cells.
-SPLIT_PASS_TRAFFIC = 175.9e6 / (256 * 384 * 256)
-SPLIT_CYCLE_TRAFFIC = (219.3e6 + 158.1e6) / (256 * 384 * 256)
+SPLIT_PASS_TRAFFIC = 173.9e6 / (256 * 384 * 256)
+SPLIT_CYCLE_TRAFFIC = (225.8e6 + 153.0e6) / (256 * 384 * 256)
 SPLIT_SOLVE_TRAFFIC = 461.5e6 / (256 * 384 * 256)
 
 

@@ -195,8 +195,9 @@ int plume_subtract_gradient(const PlumeGridInfo* info, float* u, float* v, float
                             void* stream);
 
 /* pressure.py:124-141 GaussSeidel / red_black_sweeps (red_black_sweep_kernel, colour 0 then 1 per sweep).
- * Each sweep is one launch that reads one pressure array and writes the other: `scratch` (same size as q,
- * contents ignored) is the second array; the result is always left in q. */
+ * A grid of up to about 10^5 cells is swept in place in one launch; a larger one in place, one colour per launch, or
+ * (plume_tune_solver's tiled sweeps) one launch per sweep from one pressure array into the other, `scratch` (same
+ * size as q, contents ignored). The result is always left in q. */
 int plume_red_black_sweeps(const PlumeGridInfo* info, float* q, float* scratch, const float* rhs, int32_t sweeps,
                            float relaxation, void* stream);
 
@@ -208,8 +209,9 @@ int plume_multigrid(const PlumeLevel* levels, int32_t level_count, int32_t cycle
  * `tiled_min_cells` cells sweep in shared-memory tiles (one launch per sweep), smaller levels one colour per
  * launch; the first level with at most `bottom_max_cells` cells and all coarser ones run in one launch of one
  * thread-block cluster, in its shared memory: bottom_kind 0 up to 16 CTAs, with the levels of up to about 10^5
- * cells above the bottom in the same launch (levels of at most `bottom_max_cells` in one CTA; 0: every level by
- * launches of its own); bottom_kind 1 8 CTAs from the bottom level on. Process-wide; defaults 2^40, 2048, 0. */
+ * cells above the bottom in the same launch (bottom levels of at most 512 cell pairs along z in one CTA, the others in
+ * slabs; bottom_max_cells 0: every level by launches of its own); bottom_kind 1 8 CTAs from the bottom level on.
+ * Process-wide; defaults 2^40, 2048, 0. */
 int plume_tune_solver(long long tiled_min_cells, long long bottom_max_cells, int32_t bottom_kind);
 /* The current pressure-solve strategy (the three values plume_tune_solver sets). */
 int plume_solver_tuning(long long* tiled_min_cells, long long* bottom_max_cells, int32_t* bottom_kind);
@@ -319,9 +321,12 @@ int plume_step(const PlumeStepState* state, const PlumeStepParams* params, void*
 
 /* ---- render ------------------------------------------------------------------------------------------ */
 
-/* light_volume.py:18-51 light_volume_kernel. `bricks` (optional, plume_brick_floats() floats) is scratch for a
- * map of each 4x4x4 brick's largest smoke value; with it, runs of samples whose eight corners are all <= 0 are
- * stepped over, which leaves every result bit unchanged (they add exactly 0). */
+/* light_volume.py:18-51 light_volume_kernel. `bricks` (optional, plume_brick_floats() floats) is scratch for two maps
+ * of 4x4x4 bricks, ceil(n / 4) an axis. The second half holds each brick's largest smoke value (over the brick and the
+ * next cell past it on each axis); the first half holds that value where it is > 0, and elsewhere -r, r from 0 to 3:
+ * every brick within r bricks on each axis is empty too. With them, runs of samples whose eight corners are all <= 0
+ * are stepped over, which leaves every result bit unchanged (they add exactly 0).
+ * plume_brick_floats is the size of both: twice the number of bricks. */
 long long plume_brick_floats(const int32_t shape[3]);
 int plume_light_volume(const int32_t shape[3], const void* smoke, int32_t storage, const float toward_light[3],
                        float cell_m, float opacity_per_density, float* light, float* bricks, void* stream);
@@ -329,8 +334,8 @@ int plume_light_volume(const int32_t shape[3], const void* smoke, int32_t storag
 /* plume_light_volume for a camera march of the same smoke (frame_renderer.py:53-63 prepare then march): only
  * the cells such a march reads get their light_volume_kernel value, bit for bit; every other cell gets 1.
  * A march reads the light at the corners of samples with smoke > 0, so a cell is read only when one of the 27
- * cells around it (itself included) holds smoke > 0. `bricks` is required and is left holding the smoke's brick
- * map. */
+ * cells around it (itself included) holds smoke > 0. `bricks` is required and is left holding the two
+ * maps of plume_light_volume. */
 int plume_march_light_volume(const int32_t shape[3], const void* smoke, int32_t storage, const float toward_light[3],
                              float cell_m, float opacity_per_density, float* light, float* bricks, void* stream);
 
@@ -339,14 +344,17 @@ int plume_march_light_volume(const int32_t shape[3], const void* smoke, int32_t 
 int plume_normal_field(const int32_t shape[3], const void* smoke, int32_t storage, float* blurred, float* scratch,
                        float* gradient, const float* weights_host, int32_t radius, void* stream);
 
-/* The brick map of a field (largest value of each 4x4x4 brick and the next cell past it on each axis). */
+/* The largest value of each 4x4x4 brick of a field and the next cell past it on each axis, one float a brick: half of
+ * plume_brick_floats. */
 int plume_brick_max(const int32_t shape[3], const void* field, int32_t storage, float* bricks, void* stream);
 
 /* raymarch.py:86-140 raymarch_kernel; image is (height, width, 5). gradient/light are the unused pass's
  * 1-cell stand-in when not read (frame_renderer.py:29-35). `bricks` (optional, plume_brick_floats() floats)
- * is scratch for the march's brick map of the smoke and temperature, built by this call; with it, samples with
- * no smoke skip their smoke sample and runs of samples with neither smoke nor glow are stepped over. Terms
- * that are exactly 0 are never evaluated, so the image is the same with or without it. */
+ * is scratch for the march's brick maps of the smoke and temperature, built by this call (a brick's kind: 2 for
+ * smoke plus 1 for a temperature that may glow; without either, -r as for plume_light_volume); with them, samples with
+ * no smoke skip their smoke sample and runs of samples with neither smoke nor glow are stepped over. Terms that are
+ * exactly 0 are never evaluated, so the image is the same with or without them; only outside the smoke, where the
+ * temperature is one value and also glow_start, is an ulp that a blend of it may exceed it by not taken for glow. */
 int plume_raymarch(const PlumeGridInfo* info, const void* smoke, const void* temperature, int32_t storage,
                    const float* gradient, const int32_t gradient_shape[3], const float* light,
                    const int32_t light_shape[3], const PlumeViewParams* view, const PlumeLookParams* look, float* image,

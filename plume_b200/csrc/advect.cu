@@ -612,8 +612,8 @@ __device__ __forceinline__ void march(const Args<T>& A, int seg, float* sm) {
 // every index inside the rings, and are evaluated from global memory after the block has met, if any thread has one:
 // one uniform branch per plane instead of two per element.
 //
-// Bound by shared-memory wavefronts (71% of their peak, four in ten of them bank conflicts of lanes whose samples lie in
-// different rows or planes) and instruction issue (65%; about 810 instructions a warp of elements). Measured on B200,
+// Bound by shared-memory wavefronts (65% of their peak at 128x192x128, four in ten of them bank conflicts of lanes whose
+// samples lie in different rows or planes) and instruction issue (64%; about 710 instructions for 32 elements). Measured on B200,
 // velocity advection with the traces formed one after the other, the backward one in its plane's step, against this:
 // 38x48x38 46 and 27 us, 64x96x64 84 and 59 us, 128x192x128 356 and 295 us, 256x384x256 2245 and 1975 us. Planes arrive
 // through registers: 4-byte asynchronous copies took five wavefronts each (2140 us against 2080 us at 256x384x256).
@@ -892,7 +892,8 @@ __device__ __forceinline__ void velocity_march(const Args<T>& A, int seg, float*
   }
 }
 
-// EPT elements per thread and MINB resident blocks per SM: 3 and 1 (80 registers a thread) or 2 and 2 (128).
+// EPT elements per thread and MINB resident blocks per SM: 1 and 3 (80 registers a thread, of which 272 bytes spill to 396
+// bytes of loads a thread, in float) or 2 and 2 (128 registers; 132 and 136 bytes).
 template <class T, int EPT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_mac_velocity(const __grid_constant__ Args<T> A) {
   extern __shared__ float sm[];

@@ -5,15 +5,18 @@
 // What bounds these levels is latency, not work: a colour pass of 50 thousand cells is a third of a microsecond
 // of arithmetic on a few SMs but costs a whole launch (2 to 5 us in a graph) as a kernel of its own, and a V-cycle
 // over four such levels is about forty dependent passes. So the levels' arrays stay in the shared memory of up to
-// 16 SMs and a pass ends in a cluster barrier (500 to 700 cycles) instead of a launch. Measured on B200, the solve
-// against per-colour launches with the levels of at most 2048 cells in one block: 38x48x38 (2 cycles) 107 against
-// 195 us, 48x48x48 (4 cycles) 207 against 413, 64x96x64 270 against 380, 75x113x91 455 against 750, 128x192x128
-// 610 against 729.
+// 16 SMs and a pass ends in a cluster barrier (500 to 700 cycles) instead of a launch. Measured on B200 when it was made,
+// the solve against the per-colour launches of then with the levels of at most 2048 cells in one block: 38x48x38 (2
+// cycles) 107 against 195 us, 48x48x48 (4 cycles) 207 against 413, 64x96x64 270 against 380, 75x113x91 455 against 750,
+// 128x192x128 610 against 729. The launched passes have since become as fast a level: with only the levels of at most
+// 2048 cells in the cluster, against the rule of multigrid.cu, 64x96x64 takes 290 and 275 us, 128x192x128 511 and 496,
+// 48x48x48 238 and 241, 38x48x38 131 and 141.
 //
 // What a pass then waits for is instruction fetch and dependent arithmetic: two to four warps a scheduler run
 // each phase once through and go on to the next. So the hot phases are free of branches over code that does not
 // run (missing neighbours read a float that stays 0, stores without a receiver go to floats nothing reads,
 // quotients have no slow path), loops are kept rolled, and index divisions are multiplications (Divider).
+// At 128 registers a thread it spills 40 bytes.
 // Rejected: 1024 threads with one cell each (more barrier time); one mbarrier arrival per neighbour and pass instead
 // of the cluster barrier (1.95 against 1.3 thousand cycles a pass over 6 thousand cells); a block's larger levels with
 // two cells of a colour per thread in one CTA instead of slabs.

@@ -11,8 +11,10 @@ namespace mac {
 // 1 or 2: that many elements per thread; 3: k_mac_velocity_long.
 //
 // Two elements share a tile's halo of hats and its staging between more elements, one leaves more blocks where the grid is
-// small. Measured on B200, two against one: 128x192x128 295 and 305 us, 160x240x160 (bfloat16) 512 and 550 us, 256x384x256
-// 1975 and 2104 us; 80x100x80 98 and 90 us, 64x96x64 70 and 59 us.
+// small. The line lies where two have stopped losing. Measured on B200, two against one: 64x96x64 68 and 66 us, 80x100x80
+// 97 and 95; between, by how the tiles fall: 75x113x91 103 and 108, 96x96x96 116 and 110, 96x144x96 148 and 155, 112x112x112
+// 157 and 173, 112x144x112 (1.8 million cells) 209 and 200; from two million on: 128x128x128 221 and 230, 112x168x112 239
+// and 240, 128x144x128 241 and 257, 128x192x128 306 and 320, 160x160x160 372 and 410, 256x384x256 1975 and 2104.
 //
 // The long form takes the axes whose coordinates split_bits does not cover, and a time step that is infinite or no number:
 // the other two keep a trace that leaves the staged planes inside them by giving it a zero velocity, and zero times such a

@@ -2,15 +2,18 @@
 // red-black Gauss-Seidel sweeps and multigrid V-cycles, with the reference's update order and arithmetic.
 //
 // Launch structure of one V-cycle:
-//   - each full sweep (red then black) is one launch of k_rb_sweep: a tile of 8x8x32 cells and a 2-cell halo
-//     in shared memory; red is updated on the tile and a 1-cell shell, then black on the tile, so every value
-//     equals the one the two separate colour passes produce;
+//   - each colour of a sweep is one launch, in place (k_colour_rows4, or k_colour_cells for rows that are no multiple
+//     of four cells; k_rb_split4 on a top level in colour-split storage);
 //   - the residual, its restriction to the coarse level and the zeroing of the coarse pressure are one
-//     launch (k_residual_restrict);
-//   - prolongation is folded into the first post-smoothing sweep (the tile loads q + prolong(coarse));
+//     launch (k_residual_restrict, k_residual_restrict_split);
+//   - prolongation is one launch (k_prolong_rows4, k_prolong_add_split8 and k_prolong_add_split4);
 //   - the small levels run in one launch (cluster_solve.cu): from the first of at most cluster_max_cells cells
-//     down, in the shared memory of a 16-CTA thread-block cluster, those of at most 2048 cells in one CTA of it.
-//     When that covers the whole hierarchy, all cycles are that one launch;
+//     down, in the shared memory of a 16-CTA thread-block cluster, the smallest of them (at most 512 cell pairs along z,
+//     so up to 1024 cells) in one CTA of it. When that covers the whole hierarchy, all cycles are that one launch;
+//   - levels of at least g_tiled_min_cells cells (by default none) sweep by k_rb_sweep instead, one launch a sweep: a tile
+//     of 8x8x32 cells and a 2-cell halo in shared memory; red is updated on the tile and a 1-cell shell, then black on the
+//     tile, so every value equals the one the two separate colour passes produce. Prolongation is folded into the first
+//     such sweep (the tile loads q + prolong(coarse));
 //   - the defect-correction solve's cycles, whose coarsest level is swept in double, run the levels of at most
 //     2048 cells in one 1024-thread block instead (k_block_solve).
 #include <algorithm>
@@ -39,7 +42,8 @@ constexpr int BOTTOM_WARP_PAIRS = 128;  // levels with at most this many cell pa
 // smaller ones one colour per launch; the first level of at most g_bottom_max_cells cells and everything
 // below it runs in one launch (coarse_plan).
 static long g_tiled_min_cells = 1L << 40;  // measured: per-colour sweeps win while the levels fit in L2
-// Levels of at most this many cells run in one CTA (plume_tune_solver's bottom_max_cells).
+// The bottom: the first level of at most this many cells and all below it (plume_tune_solver's bottom_max_cells). Those of at
+// most 512 cell pairs along z (cluster_solve_single) run in one CTA, larger ones in slabs.
 static long g_bottom_max_cells = 2048;
 // The top level runs in colour-split storage (given caller scratch) when it has at least this many cells
 // (plume_tune_split): levels whose q and rhs do not fit in L2. Measured on B200 at 256x384x256, 4 V-cycles: the
@@ -50,10 +54,15 @@ static long g_split_min_cells = 1L << 23;
 static int g_bottom_kind = 0;  // 0: levels above the bottom join its launch in a 16-CTA cluster; 1: an 8-CTA cluster from the bottom
 // Levels above the bottom join its launch (bottom kind 0) up to this many cells. A colour pass of a level costs a launch
 // of its own about 2 us in a graph, and in the cluster 0.6 us and 0.8 us more per 110 thousand cells; where the cluster
-// starts below the top level, each cycle also loads and stores its first level (3 us). Measured on B200, 4 cycles, with
-// the level at stake in the cluster and as launches of its own: 32x48x32 below a 64x96x64 grid 270 and 284 us,
-// 40x60x40 below 160x240x160 1147 and 1133 us, 48x72x48 below 96x144x96 468 and 439 us; the top level 48x48x48 207 and
-// 217 us, 48x72x48 236 and 229 us; overhanging cells cost the launches more: 38x57x46 below 75x113x91 455 and 482 us.
+// starts below the top level, each cycle also loads and stores its first level (3 us). Measured on B200, 4 cycles, the
+// solve with the level at stake in the cluster and as launches of its own:
+//   the top level: 40x40x40 200 and 212 us, 48x48x48 228 and 226, 75x33x45 253 and 252; 52x52x52 254 and 236, 48x72x48
+//   258 and 235;
+//   below it: 32x48x32 275 and 279 us (64x96x64 grid), 500 and 504 (128x192x128); 36x40x36 305 and 296 (72x80x72), 38x38x38
+//   684 and 679 (152x152x152), 36x48x36 336 and 322 (72x96x72), 40x60x40 960 and 938 (160x240x160);
+//   below it, with overhanging cells: 35x45x39 379 and 354 us (69x90x77), 38x57x46 425 and 389 (75x113x91), 49x49x49 458
+//   and 406 (97x97x97). Their limit dates from launched passes that branched on a cell's surroundings (482 us at 75x113x91,
+//   455 in the cluster); against the present ones, 6 to 11% faster there, it lies too high.
 // PLUME_CLUSTER_MAX_CELLS overrides both limits (for measurements).
 static long cluster_max_cells(const PlumeGridInfo& info, bool top) {
   static const long set = [] {

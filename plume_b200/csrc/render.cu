@@ -70,8 +70,8 @@ __device__ __forceinline__ float samples_within(const SkipAxis& a, float g, int 
   return unbounded ? 3.0e38f : (room - margin) * a.per_cell;
 }
 
-// Index of the sample a march continues from after the sample `s` in an empty brick: past every later sample
-// that `samples_in_brick` places in the same brick, and at most `end`.
+// Index of the sample a march continues from after the sample `s` in an empty brick: `count` samples further (those that
+// cannot leave the empty bricks around it), and at most `end`.
 __device__ __forceinline__ int past_brick(int s, int end, float count) {
   return count >= 1.0f ? s + (int)fminf(count, (float)(end - s)) : s;
 }

@@ -14,7 +14,8 @@ class LightVolume:
         self.toward_light = tuple(float(x) for x in direction / np.linalg.norm(direction))
         self.opacity_per_density = opacity_per_density
         self.light = torch.zeros(tuple(cells), dtype=torch.float32, device=device)
-        # per-frame map of each 4x4x4 brick's largest smoke value: the march skips samples that add nothing
+        # scratch for the per-frame brick map (how far each 4x4x4 brick without smoke is from the next one with some):
+        # the march skips samples that add nothing
         self.bricks = torch.empty(N.lib().plume_brick_floats(N.c_int3(*cells)), dtype=torch.float32, device=device)
 
     def compute(self, smoke: torch.Tensor, cell_m: float, march_cells: bool = False) -> torch.Tensor:

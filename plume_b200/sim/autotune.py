@@ -9,8 +9,8 @@ import torch
 
 from plume_b200.sim.multigrid import Multigrid, SolverTuning, solver_tuning, tune_solver
 
-# one-block bottom from the first level of at most 512, 2048 or 8192 cells; tiled sweeps on the largest levels
-# (at least 2^20 cells) or never; the 8-CTA cluster bottom at 2048 cells
+# the 16-CTA cluster's bottom from the first level of at most 512, 2048 or 8192 cells; tiled sweeps on the largest
+# levels (at least 2^20 cells) or never; the 8-CTA cluster from the first level of at most 2048 cells on
 DEFAULT_CANDIDATES = ((1 << 40, 2048, 0), (1 << 40, 512, 0), (1 << 40, 8192, 0), (1 << 20, 2048, 0),
                       (1 << 40, 2048, 1))
 

@@ -26,7 +26,8 @@ class SolverTuning:
     """The library's pressure-solve strategy (results do not depend on it): levels of at least
     `tiled_min_cells` cells sweep in shared-memory tiles, one launch per sweep; smaller ones one colour per
     launch; the first level of at most `bottom_max_cells` cells and all coarser ones run in one launch of one
-    thread-block cluster (`bottom_kind` 0: 16 CTAs, larger levels above the bottom in the same launch; 1: 8 CTAs)."""
+    thread-block cluster (`bottom_kind` 0: 16 CTAs, larger levels above the bottom in the same launch; 1: 8 CTAs),
+    levels of up to 512 cell pairs along z in one CTA of it."""
 
     tiled_min_cells: int
     bottom_max_cells: int
