@@ -22,7 +22,8 @@ SOURCES = [PACKAGE / "csrc" / "sim.cu", PACKAGE / "csrc" / "advect.cu", PACKAGE 
            PACKAGE / "csrc" / "view.cu", PACKAGE / "csrc" / "adjoint.cu"]
 HEADERS = [PACKAGE / "csrc" / "common.cuh", PACKAGE / "csrc" / "poisson.cuh", PACKAGE / "csrc" / "cluster_solve.cuh",
            PACKAGE / "csrc" / "stencil_table.cuh", PACKAGE / "csrc" / "advect.cuh",
-           PACKAGE / "csrc" / "light_range.cuh", PACKAGE / "csrc" / "march_plan.cuh", REPO / "include" / "plume_b200.h"]
+           PACKAGE / "csrc" / "light_range.cuh", PACKAGE / "csrc" / "march_plan.cuh",
+           PACKAGE / "csrc" / "once_per_device.cuh", REPO / "include" / "plume_b200.h"]
 LIBRARY = PACKAGE / "libplume_b200.so"
 NVCC_FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-fmad=false",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]

@@ -34,6 +34,7 @@
 
 #include "advect.cuh"
 #include "march_plan.cuh"
+#include "once_per_device.cuh"
 
 namespace plume {
 namespace mac {
@@ -972,13 +973,16 @@ static int blocks_per_sm() {
 }
 
 
+// Lets the kernel use `smem` bytes of shared memory on the current device.
 template <class Kernel>
-static int configure(Kernel k, size_t smem, bool& done) {
-  if (done) return PLUME_OK;
-  cudaError_t err = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (err != cudaSuccess) return runtime_status("fused advection: shared memory", err);
-  done = true;
-  return PLUME_OK;
+static int configure(Kernel k, size_t smem, OncePerDevice& done) {
+  int device = 0;
+  const int status = runtime_status("current device", cudaGetDevice(&device));
+  if (status != PLUME_OK) return status;
+  return done.run(device, [&] {
+    return runtime_status("fused advection: shared memory",
+                          cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  });
 }
 
 }  // namespace mac
@@ -1000,7 +1004,7 @@ long long mac_partial_floats(const PlumeGridInfo& info) {
 template <class T>
 int launch_mac_velocity(const PlumeGridInfo& info, const T* u, const T* v, const T* w, T* u_next, T* v_next,
                         T* w_next, float dt_over_cell, cudaStream_t st) {
-  static bool configured[3] = {};
+  static OncePerDevice configured[3];
   const int form = mac::march_form(info.dims, dt_over_cell, mac::env_int("PLUME_MAC_ELEMENTS")), ept = form == 2 ? 2 : 1;
   auto kernel = form == 3 ? mac::k_mac_velocity_long<T>
                           : (form == 2 ? mac::k_mac_velocity<T, 2, 2> : mac::k_mac_velocity<T, 1, 3>);
@@ -1032,7 +1036,7 @@ int launch_mac_scalars(const PlumeGridInfo& info, const T* u, const T* v, const 
                        const T* temperature, T* smoke_next, T* temperature_next, float smoke_outside,
                        float heat_outside, int uses_outside, float* seg_sums, double* line_partials, int dissipate,
                        float heat_keep, float ambient, float dt_over_cell, cudaStream_t st) {
-  static bool configured[5] = {};
+  static OncePerDevice configured[5];
   const int bps = mac::blocks_per_sm();
   auto kernel = bps == 2 ? mac::k_mac_scalars<T, 2> : (bps == 3 ? mac::k_mac_scalars<T, 3> : mac::k_mac_scalars<T, 4>);
   int status = mac::configure(kernel, mac::SCALAR_SMEM, configured[bps]);
