@@ -768,7 +768,7 @@ bool cluster_solve_runs(const ClusterSolve& s) {
   int device = 0;
   if (s.count < 1 || s.count > CLUSTER_MAX_LEVELS || cluster_solve_bytes(s) > CS_MAX_SMEM) return false;
   for (int l = 0; l < s.count; ++l)
-    if (!spacing_in_range(s.levels[l].info)) return false;
+    if (!spacing_in_range(s.levels[l].info) || (l > 0 && !halves(s.levels[l - 1].info, s.levels[l].info))) return false;
   if (s.single_from < s.count && !cluster_solve_single(s.levels[s.single_from].info)) return false;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return false;
   return s.ctas <= 8 || g_cluster_16[device];

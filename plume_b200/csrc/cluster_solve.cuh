@@ -24,6 +24,13 @@ struct ClusterSolve {
   float last_relaxation;
 };
 
+// Whether a level has half of another's cells on every axis, rounded up (multigrid.py:71-121): what the passes between two
+// levels with several cells a thread, and the cluster, are written for.
+inline bool halves(const PlumeGridInfo& fine, const PlumeGridInfo& coarse) {
+  for (int a = 0; a < 3; ++a)
+    if (coarse.dims[a] != fine.dims[a] / 2 + fine.dims[a] % 2) return false;
+  return true;
+}
 // Whether a level is small enough for one CTA (one cell of each colour per thread).
 bool cluster_solve_single(const PlumeGridInfo& info);
 // Dynamic shared memory per CTA of such a solve (bytes), and whether this device can run it.

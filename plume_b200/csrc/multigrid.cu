@@ -7,6 +7,7 @@
 //   - the residual, its restriction to the coarse level and the zeroing of the coarse pressure are one
 //     launch (k_residual_restrict, k_residual_restrict_split);
 //   - prolongation is one launch (k_prolong_rows4, k_prolong_add_split8 and k_prolong_add_split4);
+//   - between levels of which one does not halve the other, these two are k_restrict_any and k_prolong_any;
 //   - the small levels run in one launch (cluster_solve.cu): from the first of at most cluster_max_cells cells
 //     down, in the shared memory of a 16-CTA thread-block cluster, the smallest of them (at most 512 cell pairs along z,
 //     so up to 1024 cells) in one CTA of it. When that covers the whole hierarchy, all cycles are that one launch;
@@ -379,6 +380,42 @@ __global__ void k_residual_restrict(const __grid_constant__ LevelTable t, Dims f
       coarse_q[out + n] = 0.0f;
     }
   }
+}
+
+// Between levels that do not halve (a caller's own hierarchy, such as one that rounds down): residual_kernel + restrict_kernel
+// + coarse.q.zero_() and prolong_add_kernel with one cell per thread and every index held to its level, so for any two
+// sets of dims. A coarse cell without children takes 0 / 0, as the reference's average does.
+__global__ void k_restrict_any(const __grid_constant__ LevelTable t, Dims fd, const float* __restrict__ q,
+                               const float* __restrict__ rhs, Dims coarse, float* __restrict__ coarse_rhs,
+                               float* __restrict__ coarse_q) {
+  wait_for_previous_grid();
+  const int i = blockIdx.z, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= coarse.n1 || k >= coarse.n2) return;
+  const int plane = fd.n1 * fd.n2;
+  float total = 0.0f, count = 0.0f;
+#pragma unroll 1
+  for (int child = 0; child < 8; ++child) {  // in the reference's order (di, dj, dk)
+    const int fi = 2 * i + (child >> 2), fj = 2 * j + (child >> 1 & 1), fk = 2 * k + (child & 1);
+    if (fi >= fd.n0 || fj >= fd.n1 || fk >= fd.n2) continue;
+    const int c = at(fd, fi, fj, fk);
+    const float xm = fi > 0 ? __ldg(q + c - plane) : 0.0f, xp = fi < fd.n0 - 1 ? __ldg(q + c + plane) : 0.0f;
+    const float ym = fj > 0 ? __ldg(q + c - fd.n2) : 0.0f, yp = fj < fd.n1 - 1 ? __ldg(q + c + fd.n2) : 0.0f;
+    const float zm = fk > 0 ? __ldg(q + c - 1) : 0.0f, zp = fk < fd.n2 - 1 ? __ldg(q + c + 1) : 0.0f;
+    const ClassStencil& e = t.e[16 * class_of(fi, fd.n0) + 4 * class_of(fj, fd.n1) + class_of(fk, fd.n2)];
+    total = total + (__ldg(rhs + c) - quotient(coupled_sum(e, xm, xp, ym, yp, zm, zp) - e.sc * __ldg(q + c), e.inv_vc));
+    count = count + 1.0f;
+  }
+  const int out = at(coarse, i, j, k);
+  coarse_rhs[out] = total / count;
+  coarse_q[out] = 0.0f;
+}
+
+__global__ void k_prolong_any(Dims coarse, Dims fine, const float* __restrict__ cq, float* __restrict__ q) {
+  wait_for_previous_grid();
+  const int i = blockIdx.z, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= fine.n1 || k >= fine.n2) return;
+  const int c = at(fine, i, j, k);
+  q[c] = q[c] + sample_index_space(cq, coarse, prolong_point(i, j, k));
 }
 
 // ---- the top level in colour-split storage -----------------------------------------------------------------
@@ -1143,6 +1180,9 @@ static int colour_sweep(const PlumeGridInfo& info, const LevelTable& table, floa
 static int launch_restrict(const PlumeGridInfo& info, const LevelTable& table, const float* q, const float* rhs,
                            const PlumeLevel& coarse, cudaStream_t st) {
   const Dims d = dims_of(info), cd = dims_of(coarse.info);
+  if (!halves(info, coarse.info))
+    return launch_solve_kernel(k_restrict_any, cell_grid(cd.n0, cd.n1, cd.n2), cell_block(), 0, st, "residual and restriction",
+                               table, d, q, rhs, cd, coarse.rhs, coarse.q);
   const bool uniform = uniform_level(info);
   const bool wide = rows4(d, q, rhs) && (((uintptr_t)coarse.rhs | (uintptr_t)coarse.q) & 7) == 0;
   const dim3 grid(((d.n2 + 3) / 4 + TZ - 1) / TZ, (cd.n1 + TY - 1) / TY, cd.n0);
@@ -1155,6 +1195,8 @@ static int launch_restrict(const PlumeGridInfo& info, const LevelTable& table, c
 static int launch_prolong(const PlumeGridInfo& info, float* q, const float* coarse_q, const PlumeGridInfo& coarse,
                           cudaStream_t st) {
   const Dims d = dims_of(info), cd = dims_of(coarse);
+  if (!halves(info, coarse))
+    return launch_solve_kernel(k_prolong_any, cell_grid(d.n0, d.n1, d.n2), cell_block(), 0, st, "prolong", cd, d, coarse_q, q);
   const bool wide = rows4(d, q, q) && ((uintptr_t)coarse_q & 7) == 0;
   const dim3 grid(((d.n2 + 3) / 4 + TZ - 1) / TZ, (d.n1 + TY - 1) / TY, d.n0);
   return launch_solve_kernel(wide ? k_prolong_rows4<true> : k_prolong_rows4<false>, grid, cell_block(), 0, st, "prolong", cd, d, coarse_q, q);
@@ -1428,10 +1470,10 @@ static int v_cycle(const PlumeLevel* levels, int count, int index, Pressure& q, 
 }
 
 // Whether the top level runs split: scratch given, at least two levels with level 0 above the bottom (a level of
-// at most g_bottom_max_cells), uniform couplings, swept by colour (not tiled) and at least g_split_min_cells cells.
+// at most g_bottom_max_cells) and halved by level 1, uniform couplings, swept by colour (not tiled) and at least g_split_min_cells cells.
 static bool use_split(const PlumeLevel* levels, int count, int coarse_f64, const float* scratch) {
   const PlumeGridInfo& info = levels[0].info;
-  return scratch && ((uintptr_t)scratch & 15) == 0 && count >= 2 && uniform_level(info) &&
+  return scratch && ((uintptr_t)scratch & 15) == 0 && count >= 2 && uniform_level(info) && halves(info, levels[1].info) &&
          cells_of(info) >= g_split_min_cells && cells_of(info) < g_tiled_min_cells &&
          coarse_plan(levels, count, coarse_f64, 0).single_from > 0;
 }
